@@ -7,15 +7,26 @@
 // walks it.
 //
 // Work is cut into warp chunks: one warp copies one chunk in `passes`
-// passes of 32 x L words, where L (words in flight per lane: 4 for 16-byte
-// words, 8 for narrower ones) is fixed by the region's proven width and
+// passes of 32 x L words, where L is the words in flight per lane and
 // `passes` (1, 2 or 4) is chosen per region class.  Warps take chunks
-// warp_id, warp_id + total warps, ... with no CTA-wide barrier; each finds
-// its chunk's region by ballot rounds over the table's first-chunk column.
-// A table of up to kSmemTableBytes is copied into shared memory once per
-// CTA (one round trip), so those lookups never touch global memory.  Each
-// region keeps its own geometry and proven vector width, so a 16-B row face
-// and a 2-KiB row face run at their own width inside the same launch.
+// warp_id, warp_id + total warps, ... with no CTA-wide barrier between
+// chunks; each finds its chunk's region by ballot rounds over the table's
+// first-chunk column, kept in shared memory.  Each region keeps its own
+// geometry and proven vector width, so a 16-B row face and a 2-KiB row face
+// run at their own width inside the same launch.
+//
+// Two sets of kernels do this.  Batches whose regions all have at most two
+// strided dimensions (every region of a grid) run the compact ones
+// (k_batch_small, k_batch_copy_small and their _param forms): 64-byte
+// entries, words reached by stepping their digits instead of dividing, 64
+// registers.  What bounds them is the rate of scattered lines for the x faces
+// (about 41 G lines/s measured by a one-load gather) and, for small halos,
+// the launch itself.  Measured against the other set on B200, launches back to
+// back over rotating buffers, pack / unpack / exchange in us: 8 mixed grids
+// (208 regions, 16.8 MB) 24.0 / 17.6 / 28.8 before, 13.5 / 14.2 / 16.7 now;
+// 320 x 300 x 310 doubles radius 3 12.4 / 12.5 / 17.5 before, 10.5 / 8.6 /
+// 10.6 now.  The others (k_batch, k_batch_copy) divide every word's index
+// over any number of dimensions, at 80 registers.
 //
 // The passes of each region class (width x words per row) and the launch
 // shape of a batch (threads per CTA, CTAs per SM) come from defaults or from
@@ -52,11 +63,15 @@ constexpr int kSmemTableBytes = 32768; // tables up to this size are staged
 constexpr int kClasses = 40;           // 5 widths x 8 row-length buckets
 constexpr int kPassChoices[3] = {1, 2, 4};
 
-// words each lane keeps in flight in one pass: 64 bytes for 8- and 16-byte
-// words (registers allow no more), 8 words for narrower ones
+// Words each lane keeps in flight in one pass.  The compact kernels take 4 of
+// any width: 64 registers, so 32 warps an SM, whose lanes' 4 requests are more
+// than DRAM takes for short rows, and whose chunks are small enough to spread
+// over all warps.  The kernels for any number of dimensions take 64 bytes for
+// 8- and 16-byte words (registers allow no more), 8 words for narrower ones.
+constexpr int kSmallWords = 4;
 template <int W> constexpr int lane_words() { return W == 16 ? 4 : 8; }
-__host__ __device__ constexpr uint32_t lane_words_of(uint32_t w) {
-  return w == 16 ? 4u : 8u;
+__host__ __device__ constexpr uint32_t lane_words_of(uint32_t w, bool small) {
+  return small ? uint32_t(kSmallWords) : w == 16 ? 4u : 8u;
 }
 
 struct BatchRegion {
@@ -78,6 +93,70 @@ struct CopyPair {
 // the geometry that sets a record's words and class
 const Geometry &geometry_of(const BatchRegion &r) { return r.g; }
 const Geometry &geometry_of(const CopyPair &r) { return r.gs; }
+
+// One strided side of a compact record: at most two strided dimensions (the
+// regions of a grid never have more once contiguous ones are merged), word
+// divisors, and what a step of 32 words adds to the digits of a word.
+struct Side {
+  char *base;           // origin + start
+  int64_t s0, s1;       // strides of the two dimensions (0: unused)
+  uint32_t wpr, wm;     // words per row and their FastDiv multiplier
+  uint32_t c0, cm;      // count of dimension 0 and its FastDiv multiplier
+  uint8_t ws, cs;       // the FastDiv shifts
+  uint8_t dcol, ddig, dq; // 32 words = dq x c0 + ddig rows and dcol words
+  uint8_t lwidth;       // log2 of the word's bytes
+  uint8_t passes;       // passes of a warp over one chunk: 1, 2 or 4
+  uint8_t spare;
+};
+
+// What the kernels read for a region or pair of at most two strided
+// dimensions: 64 and 104 bytes instead of 168 and 288, so a halo's 26 regions
+// take 2 KB of kernel parameters and one entry two sectors.
+struct SmallRegion {
+  Side s;
+  char *packed;
+  uint32_t total_words;
+  uint32_t chunk_begin;
+};
+
+struct SmallPair {
+  Side s, d; // s.passes and s.lwidth hold for both
+  uint32_t total_words;
+  uint32_t chunk_begin;
+};
+static_assert(sizeof(Side) == 48 && sizeof(SmallRegion) == 64 &&
+                  sizeof(SmallPair) == 104,
+              "record sizes are documented");
+
+Side make_side(const char *base, const Geometry &g, uint32_t passes) {
+  Side s{};
+  s.base = const_cast<char *>(base);
+  s.s0 = g.strides[0];
+  s.s1 = g.strides[1];
+  s.wpr = g.wpr;
+  s.wm = g.wdiv.m;
+  s.ws = uint8_t(g.wdiv.s);
+  s.c0 = std::max(1u, g.cdiv[0].d);
+  s.cm = g.cdiv[0].m;
+  s.cs = uint8_t(g.cdiv[0].s);
+  const uint32_t drow = 32 / s.wpr;
+  s.dcol = uint8_t(32 - drow * s.wpr);
+  s.dq = uint8_t(drow / s.c0);
+  s.ddig = uint8_t(drow % s.c0);
+  s.lwidth = uint8_t(31 - __builtin_clz(g.width));
+  s.passes = uint8_t(passes);
+  return s;
+}
+bool is_small(const BatchRegion &r) { return r.g.nd <= 2; }
+bool is_small(const CopyPair &r) { return r.gs.nd <= 2 && r.gd.nd <= 2; }
+SmallRegion make_small(const BatchRegion &r) {
+  return {make_side(r.strided, r.g, r.passes), r.packed, r.g.total_words,
+          r.chunk_begin};
+}
+SmallPair make_small(const CopyPair &r) {
+  return {make_side(r.src, r.gs, r.passes), make_side(r.dst, r.gd, r.passes),
+          r.gs.total_words, r.chunk_begin};
+}
 
 template <int W> struct BWord;
 template <> struct BWord<1> { using T = uint8_t; };
@@ -197,15 +276,16 @@ __device__ __forceinline__ void copy_chunk_p(const CopyPair &r, uint32_t c,
 // Index of the last entry whose first chunk is <= chunk, found by one warp:
 // each round the lanes sample 32 evenly spaced entries of the remaining
 // stretch and a ballot narrows it 32-fold, so n entries take ceil(log32 n)
-// rounds (one for a 26-region halo, two for up to 1024 regions).
-template <typename Rec>
-__device__ __forceinline__ int find_region(const Rec *r, int n, uint32_t chunk,
+// rounds (one for a 26-region halo, two for up to 1024 regions).  `begin(i)`
+// is entry i's first chunk.
+template <typename Begin>
+__device__ __forceinline__ int find_region(Begin begin, int n, uint32_t chunk,
                                            uint32_t lane) {
   int base = 0, len = n;
   while (true) {
     const int step = (len + 31) / 32;
     const int off = int(lane) * step;
-    const bool le = off < len && r[base + off].chunk_begin <= chunk;
+    const bool le = off < len && begin(base + off) <= chunk;
     const unsigned m = __ballot_sync(0xffffffffu, le);
     const int seg = 31 - __clz(m); // the stretch's first entry always qualifies
     base += seg * step;
@@ -242,7 +322,8 @@ __device__ __forceinline__ void batch_chunks(const BatchRegion *tab,
   const uint32_t nwarps = gridDim.x * (THREADS / 32);
   for (uint32_t c = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
        c < total_chunks; c += nwarps) {
-    const BatchRegion &r = tab[find_region(tab, nregions, c, lane)];
+    const BatchRegion &r = tab[find_region([&](int i) { return tab[i].chunk_begin; },
+                                           nregions, c, lane)];
     switch (r.g.width) {
     case 16: pack_chunk_p<16>(r, c, lane, unpack); break;
     case 8: pack_chunk_p<8>(r, c, lane, unpack); break;
@@ -275,7 +356,8 @@ __global__ void __launch_bounds__(THREADS, (768 + THREADS - 1) / THREADS)
   const uint32_t nwarps = gridDim.x * (THREADS / 32);
   for (uint32_t c = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
        c < total_chunks; c += nwarps) {
-    const CopyPair &r = tab[find_region(tab, npairs, c, lane)];
+    const CopyPair &r = tab[find_region([&](int i) { return tab[i].chunk_begin; },
+                                        npairs, c, lane)];
     switch (r.gs.width) {
     case 16: copy_chunk_p<16>(r, c, lane); break;
     case 8: copy_chunk_p<8>(r, c, lane); break;
@@ -284,6 +366,169 @@ __global__ void __launch_bounds__(THREADS, (768 + THREADS - 1) / THREADS)
     default: copy_chunk_p<1>(r, c, lane); break;
     }
   }
+}
+
+// ---- records of at most two strided dimensions -----------------------------
+
+// Strided-side offsets of the words w, w + 32, w + 64, ... of a Side, for one
+// lane: a word is (column, digit of dimension 0, digit of dimension 1), and a
+// step of 32 words adds fixed amounts to the digits with at most one carry
+// each, so a step is two compares and three 64-bit adds, where dividing every
+// word anew took about 40 instructions and twice the registers.
+struct Walk {
+  int64_t off;
+  uint32_t col, dig;         // column in words, digit of dimension 0
+  uint32_t wpr, c0;          // their limits
+  uint32_t dcol, ddig;       // added to them by a step
+  int64_t step, wrap, carry; // added to off: by a step, when the column
+                             // passes the row's end, when the digit passes c0
+
+  __device__ __forceinline__ Walk(uint32_t w, const Side &g) {
+    const int64_t s0 = g.s0, s1 = g.s1;
+    const uint32_t lw = g.lwidth;
+    wpr = g.wpr;
+    c0 = g.c0;
+    dcol = g.dcol;
+    ddig = g.ddig;
+    const uint32_t row = g.wm ? __umulhi(w, g.wm) >> g.ws : w;
+    const uint32_t q = g.cm ? __umulhi(row, g.cm) >> g.cs : row;
+    col = w - row * wpr;
+    dig = row - q * c0;
+    off = int64_t(q) * s1 + int64_t(dig) * s0 + int64_t(col << lw);
+    step = int64_t(g.dq) * s1 + int64_t(ddig) * s0 + int64_t(dcol << lw);
+    wrap = s0 - (int64_t(wpr) << lw);
+    carry = s1 - int64_t(c0) * s0;
+  }
+  __device__ __forceinline__ void next() {
+    off += step;
+    col += dcol;
+    dig += ddig;
+    if (col >= wpr) {
+      col -= wpr;
+      ++dig;
+      off += wrap;
+    }
+    if (dig >= c0) {
+      dig -= c0;
+      off += carry;
+    }
+  }
+};
+
+// One pass of a warp over U x 32 words of a region: words w, w + 32, ... with
+// `left` > 0 words (signed) from w to the region's end.  U loads are in
+// flight per lane; offsets are walked, never held.
+template <int W, int U, bool UNPACK>
+__device__ __forceinline__ void move_words(const SmallRegion &r, uint32_t w,
+                                           int left) {
+  using T = typename BWord<W>::T;
+  char *strided = r.s.base;
+  T *packed = reinterpret_cast<T *>(r.packed) + w;
+  Walk at(w, r.s);
+  T v[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (32 * u < left)
+      v[u] = __ldg(UNPACK ? packed + 32 * u
+                          : reinterpret_cast<const T *>(strided + at.off));
+    if (!UNPACK)
+      at.next();
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (32 * u < left)
+      *(UNPACK ? reinterpret_cast<T *>(strided + at.off) : packed + 32 * u) = v[u];
+    if (UNPACK)
+      at.next();
+  }
+}
+
+// one pass over a copy pair: the loads at the source side first, then the
+// stores at the destination side
+template <int W, int U, bool UNPACK>
+__device__ __forceinline__ void move_words(const SmallPair &r, uint32_t w,
+                                           int left) {
+  using T = typename BWord<W>::T;
+  T v[U];
+  {
+    const char *src = r.s.base;
+    Walk at(w, r.s);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (32 * u < left)
+        v[u] = __ldg(reinterpret_cast<const T *>(src + at.off));
+      at.next();
+    }
+  }
+  char *dst = r.d.base;
+  Walk at(w, r.d);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (32 * u < left)
+      *reinterpret_cast<T *>(dst + at.off) = v[u];
+    at.next();
+  }
+}
+
+// Every warp chunk of the table `tab`, warps taking chunks warp_id,
+// warp_id + total warps, ...  The searches read the first-chunk column from
+// `s_begin` (shared memory, filled here once per CTA) when `staged`, else
+// from the table; the entries themselves are read in place, each field once
+// per pass with one address for all lanes.
+template <bool UNPACK, typename Rec>
+__device__ __forceinline__ void small_chunks(const Rec *tab, int n,
+                                             uint32_t total_chunks, int staged,
+                                             uint32_t *s_begin) {
+  if (staged) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      s_begin[i] = tab[i].chunk_begin;
+    __syncthreads();
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+#pragma unroll 1
+  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+       c < total_chunks; c += nwarps) {
+    const int at =
+        staged ? find_region([&](int i) { return s_begin[i]; }, n, c, lane)
+               : find_region([&](int i) { return tab[i].chunk_begin; }, n, c, lane);
+    const uint32_t lw = tab[at].s.lwidth, passes = tab[at].s.passes;
+    constexpr uint32_t per = 32 * kSmallWords;
+    uint32_t w = (c - tab[at].chunk_begin) * passes * per + lane;
+#pragma unroll 1
+    for (uint32_t p = 0; p < passes; ++p, w += per) {
+      const Rec &r = tab[at];
+      const int left = int(r.total_words - w);
+      if (left <= 0)
+        break;
+      switch (lw) {
+      case 4: move_words<16, kSmallWords, UNPACK>(r, w, left); break;
+      case 3: move_words<8, kSmallWords, UNPACK>(r, w, left); break;
+      case 2: move_words<4, kSmallWords, UNPACK>(r, w, left); break;
+      case 1: move_words<2, kSmallWords, UNPACK>(r, w, left); break;
+      default: move_words<1, kSmallWords, UNPACK>(r, w, left); break;
+      }
+    }
+  }
+}
+
+constexpr int kSmallThreadsPerSm = 1024;
+template <int THREADS, bool UNPACK>
+__global__ void
+__launch_bounds__(THREADS, kSmallThreadsPerSm / THREADS)
+    k_batch_small(const SmallRegion *__restrict__ regions, int nregions,
+                  uint32_t total_chunks, int staged) {
+  extern __shared__ __align__(16) uint32_t s_begin[];
+  small_chunks<UNPACK>(regions, nregions, total_chunks, staged, s_begin);
+}
+
+template <int THREADS>
+__global__ void
+__launch_bounds__(THREADS, kSmallThreadsPerSm / THREADS)
+    k_batch_copy_small(const SmallPair *__restrict__ pairs, int npairs,
+                       uint32_t total_chunks, int staged) {
+  extern __shared__ __align__(16) uint32_t s_begin[];
+  small_chunks<false>(pairs, npairs, total_chunks, staged, s_begin);
 }
 
 // read every 16-B word of a buffer larger than the L2 (the autotuner's
@@ -321,29 +566,41 @@ struct Shape {
   int ctas_per_sm = 0; // 0: as many as fit
 };
 
+// the batch kernels: what they do (rows) at 128, 256 and 512 threads; the
+// first three take compact records, the others any number of dimensions
+enum { kSmallPack, kSmallUnpack, kSmallCopy, kAnyPack, kAnyCopy };
+const void *batch_kernel(int kind, int threads) {
+  static const void *fns[5][3] = {
+      {(const void *)k_batch_small<128, false>,
+       (const void *)k_batch_small<256, false>,
+       (const void *)k_batch_small<512, false>},
+      {(const void *)k_batch_small<128, true>,
+       (const void *)k_batch_small<256, true>,
+       (const void *)k_batch_small<512, true>},
+      {(const void *)k_batch_copy_small<128>,
+       (const void *)k_batch_copy_small<256>,
+       (const void *)k_batch_copy_small<512>},
+      {(const void *)k_batch<128>, (const void *)k_batch<256>,
+       (const void *)k_batch<512>},
+      {(const void *)k_batch_copy<128>, (const void *)k_batch_copy<256>,
+       (const void *)k_batch_copy<512>}};
+  return fns[kind][threads == 128 ? 0 : threads == 512 ? 2 : 1];
+}
+
 // how many CTAs of a batch kernel fit one SM (cached per kernel and size)
-int max_ctas(bool copy, int threads, int smem) {
+int max_ctas(int kind, int threads, int smem) {
   static std::mutex mu;
-  static std::map<std::tuple<bool, int, int, int>, int> cache;
+  static std::map<std::tuple<int, int, int, int>, int> cache;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> l(mu);
-  auto key = std::make_tuple(copy, threads, smem, dev);
+  auto key = std::make_tuple(kind, threads, smem, dev);
   auto it = cache.find(key);
   if (it != cache.end())
     return it->second;
-  const void *fn = nullptr;
-  if (copy)
-    fn = threads == 128   ? (const void *)k_batch_copy<128>
-         : threads == 512 ? (const void *)k_batch_copy<512>
-                          : (const void *)k_batch_copy<256>;
-  else
-    fn = threads == 128   ? (const void *)k_batch<128>
-         : threads == 512 ? (const void *)k_batch<512>
-                          : (const void *)k_batch<256>;
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) !=
-          cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &n, batch_kernel(kind, threads), threads, smem) != cudaSuccess ||
       n < 1) {
     cudaGetLastError();
     n = 1;
@@ -352,57 +609,73 @@ int max_ctas(bool copy, int threads, int smem) {
   return n;
 }
 
+uint64_t chunks_of(const Geometry &g, uint32_t passes, bool small) {
+  const uint64_t per = 32ull * lane_words_of(g.width, small) * passes;
+  return (g.total_words + per - 1) / per;
+}
+
+// Whether a batch takes the compact kernels: every entry fits a compact
+// record, and its chunks, up to twice as many as the other kernels cut, can
+// be counted in 32 bits even at one pass each (so that no tuning of the
+// passes changes the answer).
+template <typename Rec> bool all_small(const std::vector<Rec> &recs) {
+  uint64_t chunks = 0;
+  for (const Rec &r : recs) {
+    chunks += chunks_of(geometry_of(r), 1, true);
+    if (!is_small(r) || chunks > UINT32_MAX)
+      return false;
+  }
+  return true;
+}
+
 // warp chunks of every record, in order; the total (or more than
 // UINT32_MAX when the batch is too large)
 template <typename Rec> uint64_t assign_chunks(std::vector<Rec> &recs) {
+  const bool small = all_small(recs);
   uint64_t chunks = 0;
   for (Rec &r : recs) {
     const Geometry &g = geometry_of(r);
     r.chunk_begin = uint32_t(std::min<uint64_t>(chunks, UINT32_MAX));
-    const uint64_t per = 32ull * lane_words_of(g.width) * r.passes;
-    chunks += (g.total_words + per - 1) / per;
+    chunks += chunks_of(g, r.passes, small);
   }
   return chunks;
 }
 
 } // namespace
 
+template <typename Rec> static int kind_of(bool small, int unpack) {
+  if (std::is_same<Rec, CopyPair>::value)
+    return small ? kSmallCopy : kAnyCopy;
+  return !small ? kAnyPack : unpack ? kSmallUnpack : kSmallPack;
+}
+
 // Launch the pack kernel (or, for pairs, the copy kernel) over a table in
-// device memory on `s`.
+// device memory on `s`: compact entries when `small`.
 template <typename Rec>
-static int launch_table(const Rec *table, int n, uint32_t total_chunks,
-                        int unpack, Shape shape, cudaStream_t s) {
+static int launch_table(const void *table, int n, bool small,
+                        uint32_t total_chunks, int unpack, Shape shape,
+                        cudaStream_t s) {
   constexpr bool kCopy = std::is_same<Rec, CopyPair>::value;
   if (n <= 0 || total_chunks == 0)
     return TEMPI_OK;
-  const int smem_need = n * int(sizeof(Rec));
-  const int staged = smem_need <= kSmemTableBytes ? 1 : 0;
+  const int smem_need = n * int(small ? sizeof(uint32_t) : sizeof(Rec));
+  int staged = smem_need <= kSmemTableBytes ? 1 : 0;
   const int smem = staged ? smem_need : 0;
   const int threads = shape.threads == 128 || shape.threads == 512
                           ? shape.threads
                           : 256;
-  const int fit = max_ctas(kCopy, threads, smem);
+  const int kind = kind_of<Rec>(small, unpack);
+  const int fit = max_ctas(kind, threads, smem);
   const int per_sm = shape.ctas_per_sm > 0 ? std::min(shape.ctas_per_sm, fit)
                                            : fit;
   const uint32_t warps_per_cta = uint32_t(threads / 32);
   const uint32_t want = (total_chunks + warps_per_cta - 1) / warps_per_cta;
   const uint32_t grid = std::max<uint32_t>(
       1, std::min<uint32_t>(want, uint32_t(num_sms()) * uint32_t(per_sm)));
-  if constexpr (kCopy) {
-    if (threads == 128)
-      k_batch_copy<128><<<grid, 128, smem, s>>>(table, n, total_chunks, staged);
-    else if (threads == 512)
-      k_batch_copy<512><<<grid, 512, smem, s>>>(table, n, total_chunks, staged);
-    else
-      k_batch_copy<256><<<grid, 256, smem, s>>>(table, n, total_chunks, staged);
-  } else {
-    if (threads == 128)
-      k_batch<128><<<grid, 128, smem, s>>>(table, n, total_chunks, unpack, staged);
-    else if (threads == 512)
-      k_batch<512><<<grid, 512, smem, s>>>(table, n, total_chunks, unpack, staged);
-    else
-      k_batch<256><<<grid, 256, smem, s>>>(table, n, total_chunks, unpack, staged);
-  }
+  void *general[] = {&table, &n, &total_chunks, &unpack, &staged};
+  void *others[] = {&table, &n, &total_chunks, &staged};
+  cudaLaunchKernel(batch_kernel(kind, threads), dim3(grid), dim3(threads),
+                   kind == kAnyPack ? general : others, size_t(smem), s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return cuda_error(e, kCopy ? "copy batch launch" : "batch launch");
@@ -491,9 +764,11 @@ uint64_t apply_passes(std::vector<Rec> &recs, const Tuned *t) {
 
 struct BatchImpl {
   std::vector<BatchRegion> host;
-  BatchRegion *dev = nullptr;
   std::vector<CopyPair> host_pairs; // a copy batch
-  CopyPair *dev_pairs = nullptr;
+  void *dev = nullptr; // the table: compact entries when `small`
+  bool small = false;
+  std::vector<SmallRegion> host_small; // the table of a small pack batch
+  std::vector<SmallPair> host_pairs_small; // and of a small copy batch
   uint32_t total_chunks = 0;
   int unpack = 0;
   Shape shape;
@@ -531,7 +806,17 @@ static uint64_t plan_batch(BatchImpl &bi, std::vector<Rec> &recs) {
 }
 
 template <typename Rec>
-static int upload(const std::vector<Rec> &recs, Rec **dev) {
+static std::vector<decltype(make_small(std::declval<Rec>()))>
+small_table(const std::vector<Rec> &recs) {
+  std::vector<decltype(make_small(std::declval<Rec>()))> t;
+  t.reserve(recs.size());
+  for (const Rec &r : recs)
+    t.push_back(make_small(r));
+  return t;
+}
+
+template <typename Rec>
+static int upload(const std::vector<Rec> &recs, void **dev) {
   if (recs.empty())
     return TEMPI_OK;
   const size_t bytes = recs.size() * sizeof(Rec);
@@ -543,6 +828,22 @@ static int upload(const std::vector<Rec> &recs, Rec **dev) {
   if (e != cudaSuccess)
     return cuda_error(e, "batch table upload");
   return TEMPI_OK;
+}
+
+// the batch's table, as its kernels read it, into device memory
+static int upload_table(BatchImpl &bi) {
+  if (!bi.host_pairs.empty()) {
+    bi.small = all_small(bi.host_pairs);
+    if (!bi.small)
+      return upload(bi.host_pairs, &bi.dev);
+    bi.host_pairs_small = small_table(bi.host_pairs);
+    return upload(bi.host_pairs_small, &bi.dev);
+  }
+  bi.small = all_small(bi.host);
+  if (!bi.small)
+    return upload(bi.host, &bi.dev);
+  bi.host_small = small_table(bi.host);
+  return upload(bi.host_small, &bi.dev);
 }
 
 extern "C" int tempi_batch_create(const tempi_region *regions, int32_t n,
@@ -575,7 +876,7 @@ extern "C" int tempi_batch_create(const tempi_region *regions, int32_t n,
     return set_error(TEMPI_ERR_ARG, "batch too large");
   }
   b->impl.total_chunks = uint32_t(chunks);
-  int err = upload(b->impl.host, &b->impl.dev);
+  int err = upload_table(b->impl);
   if (err) {
     cudaFree(b->impl.dev);
     delete b;
@@ -585,16 +886,15 @@ extern "C" int tempi_batch_create(const tempi_region *regions, int32_t n,
   return TEMPI_OK;
 }
 
-template <int P> struct StaticPiece {
-  BatchRegion r[P];
+template <int P, typename Rec = BatchRegion> struct StaticPiece {
+  Rec r[P];
 };
 
 // A batch of up to kParamRegions regions in one launch with its table in the
-// kernel's parameters (5.4 KB): each CTA copies it from there into shared
-// memory instead of from global memory.  Used by the allocation-free entry
-// point (neither a fill kernel nor the fixed array is involved) and by
-// small batches at the default launch shape.  256 threads, 3 CTAs per SM by
-// the launch bounds.
+// kernel's parameters (2 KB of compact entries, or 5.4 KB for more than two
+// strided dimensions), read there in place.  Used by the allocation-free
+// entry point (neither a fill kernel nor the fixed array is involved) and by
+// small batches at the default launch shape.
 constexpr int kParamRegions = 32;
 
 template <int P>
@@ -606,22 +906,55 @@ __global__ void __launch_bounds__(256, 3)
   batch_chunks<256>(piece.r, nregions, total_chunks, unpack);
 }
 
-// k_batch_param over `n` <= kParamRegions entries of `table` (host memory),
-// `per_sm` CTAs per SM (at most 3)
-static int launch_param(const BatchRegion *table, int n, uint32_t total_chunks,
+template <int P, bool UNPACK>
+__global__ void __launch_bounds__(256, kSmallThreadsPerSm / 256)
+    k_batch_param_small(const __grid_constant__ StaticPiece<P, SmallRegion> piece,
+                        int nregions, uint32_t total_chunks) {
+  __shared__ uint32_t s_begin[P];
+  small_chunks<UNPACK>(piece.r, nregions, total_chunks, 1, s_begin);
+}
+
+template <int P>
+__global__ void __launch_bounds__(256, kSmallThreadsPerSm / 256)
+    k_batch_copy_param(const __grid_constant__ StaticPiece<P, SmallPair> piece,
+                       int npairs, uint32_t total_chunks) {
+  __shared__ uint32_t s_begin[P];
+  small_chunks<false>(piece.r, npairs, total_chunks, 1, s_begin);
+}
+
+// k_batch_param(_small) over the `n` <= kParamRegions entries of `table`
+// (host memory), `per_sm` CTAs per SM (0: as many as fit)
+template <typename Rec>
+static int launch_param(const Rec *table, int n, uint32_t total_chunks,
                         int unpack, int per_sm, cudaStream_t s) {
-  StaticPiece<kParamRegions> piece;
-  std::memcpy(piece.r, table, size_t(n) * sizeof(BatchRegion));
+  constexpr bool kSmall = !std::is_same<Rec, BatchRegion>::value;
+  StaticPiece<kParamRegions, Rec> piece;
+  std::memcpy(piece.r, table, size_t(n) * sizeof(Rec));
+  const int fit = kSmall ? kSmallThreadsPerSm / 256 : 3; // by the launch bounds
+  per_sm = per_sm > 0 ? std::min(per_sm, fit) : fit;
   const uint32_t grid = std::max<uint32_t>(
       1, std::min<uint32_t>((total_chunks + 7) / 8,
                             uint32_t(num_sms()) * uint32_t(per_sm)));
-  k_batch_param<kParamRegions><<<grid, 256, 0, s>>>(piece, n, total_chunks,
-                                                     unpack);
+  if constexpr (!kSmall)
+    k_batch_param<kParamRegions><<<grid, 256, 0, s>>>(piece, n, total_chunks,
+                                                       unpack);
+  else if constexpr (std::is_same<Rec, SmallPair>::value)
+    k_batch_copy_param<kParamRegions><<<grid, 256, 0, s>>>(piece, n, total_chunks);
+  else if (unpack)
+    k_batch_param_small<kParamRegions, true><<<grid, 256, 0, s>>>(piece, n, total_chunks);
+  else
+    k_batch_param_small<kParamRegions, false><<<grid, 256, 0, s>>>(piece, n, total_chunks);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return cuda_error(e, "batch launch");
   counters().kernel_launches++;
   return TEMPI_OK;
+}
+
+// whether a launch shape is one that the parameter kernels can take
+static bool param_shape(const Shape &shape, bool small) {
+  return (shape.threads == 0 || shape.threads == 256) &&
+         (small || shape.ctas_per_sm <= 3);
 }
 
 // `direct`: a launch of its own (tempi_batch_launch).  There a small table at
@@ -632,21 +965,29 @@ static int launch_param(const BatchRegion *table, int n, uint32_t total_chunks,
 // replayed kernel node with 5.4 KB of parameters measured 1-2 us slower.
 static int batch_launch(tempi_batch *b, cudaStream_t s, bool direct) {
   BatchImpl &bi = b->impl;
-  if (!bi.host_pairs.empty())
-    return launch_table(bi.dev_pairs, int(bi.host_pairs.size()),
-                        bi.total_chunks, 0, bi.shape, s);
-  const int n = int(bi.host.size());
+  const bool copy = !bi.host_pairs.empty();
+  const int n = int(copy ? bi.host_pairs.size() : bi.host.size());
   if (direct && n > 0 && n <= kParamRegions && bi.total_chunks > 0 &&
-      (bi.shape.threads == 0 || bi.shape.threads == 256) &&
-      bi.shape.ctas_per_sm <= 3) {
-    const int per_sm = bi.shape.ctas_per_sm > 0 ? bi.shape.ctas_per_sm : 3;
-    const int err = launch_param(bi.host.data(), n, bi.total_chunks, bi.unpack,
-                                 per_sm, s);
+      param_shape(bi.shape, bi.small) && (bi.small || !copy)) {
+    const int per_sm = bi.shape.ctas_per_sm;
+    const int err =
+        copy ? launch_param(bi.host_pairs_small.data(), n, bi.total_chunks, 0,
+                            per_sm, s)
+        : bi.small ? launch_param(bi.host_small.data(), n, bi.total_chunks,
+                                  bi.unpack, per_sm, s)
+                   : launch_param(bi.host.data(), n, bi.total_chunks,
+                                  bi.unpack, per_sm, s);
     if (!err)
-      set_last_kernel(bi.unpack ? "batch_unpack" : "batch_pack");
+      set_last_kernel(copy        ? "batch_copy"
+                      : bi.unpack ? "batch_unpack"
+                                  : "batch_pack");
     return err;
   }
-  return launch_table(bi.dev, n, bi.total_chunks, bi.unpack, bi.shape, s);
+  if (copy)
+    return launch_table<CopyPair>(bi.dev, n, bi.small, bi.total_chunks, 0,
+                                  bi.shape, s);
+  return launch_table<BatchRegion>(bi.dev, n, bi.small, bi.total_chunks,
+                                   bi.unpack, bi.shape, s);
 }
 
 // Copy pairs for `regions`, each at the default passes of its class; empty
@@ -674,9 +1015,10 @@ static int build_pairs(const tempi_copy_region *regions, int32_t n,
                           &cp.gd, &ed);
     if (!err && !es && !ed) {
       const int w = int(std::min(cp.gs.width, cp.gd.width));
-      err = make_geometry(&r.src_desc, r.src_count, uintptr_t(src), 0, w,
-                          &cp.gs, &es);
-      if (!err)
+      if (int(cp.gs.width) != w)
+        err = make_geometry(&r.src_desc, r.src_count, uintptr_t(src), 0, w,
+                            &cp.gs, &es);
+      if (int(cp.gd.width) != w)
         err = make_geometry(&r.dst_desc, r.dst_count, uintptr_t(dst), 0, w,
                             &cp.gd, &ed);
     }
@@ -712,10 +1054,10 @@ extern "C" int tempi_batch_create_copy(const tempi_copy_region *regions,
   }
   if (!err) {
     b->impl.total_chunks = uint32_t(chunks);
-    err = upload(b->impl.host_pairs, &b->impl.dev_pairs);
+    err = upload_table(b->impl);
   }
   if (err) {
-    cudaFree(b->impl.dev_pairs);
+    cudaFree(b->impl.dev);
     delete b;
     return err;
   }
@@ -725,61 +1067,64 @@ extern "C" int tempi_batch_create_copy(const tempi_copy_region *regions,
 
 namespace tempi {
 
-// One copy batch on `s` with the pair table in a grow-only device buffer:
-// no allocation once the buffer is large enough.  The caller synchronises
-// `s` before the next call (the table is rewritten by every call).
+// One copy batch on `s`.  Up to kParamRegions pairs of at most two strided
+// dimensions (a halo's 26) travel in the kernel's parameters: nothing is
+// uploaded, whatever regions the previous call had.  Larger tables go to a
+// grow-only device buffer: no allocation once it is large enough.  The caller
+// synchronises `s` before the next call (the table is rewritten by every
+// call).
 int copy_batch_run(const tempi_copy_region *regions, int32_t n,
                    cudaStream_t s) {
   static std::mutex mu;
-  static CopyPair *table = nullptr;
-  static size_t capacity = 0;
-  static std::vector<CopyPair> pairs, on_device;
-  static Shape shape;
-  static uint64_t on_device_sig = 0;
+  static void *table = nullptr;
+  static size_t capacity = 0; // bytes
+  static std::vector<CopyPair> pairs;
   std::lock_guard<std::mutex> l(mu);
   uint64_t chunks = 0;
   int err = build_pairs(regions, n, &pairs, &chunks);
   if (err || pairs.empty())
     return err;
   // a batch of a tuned signature takes the tuned choices
-  const uint64_t sig = signature(pairs, 0);
-  if (sig != on_device_sig || on_device.size() != pairs.size()) {
+  Shape shape;
+  {
     std::lock_guard<std::mutex> t(g_tune_mu);
     load_tuned_locked();
-    auto it = g_tuned.find(sig);
-    shape = it != g_tuned.end() ? it->second.shape : Shape{};
-    if (it != g_tuned.end())
+    auto it = g_tuned.empty() ? g_tuned.end() : g_tuned.find(signature(pairs, 0));
+    if (it != g_tuned.end()) {
+      shape = it->second.shape;
       chunks = apply_passes(pairs, &it->second);
-  } else {
-    // same signature as the table on the device: same choices
-    for (size_t i = 0; i < pairs.size(); ++i)
-      pairs[i].passes = on_device[i].passes;
-    chunks = assign_chunks(pairs);
+    }
   }
-  if (pairs.size() > capacity) {
+  const int count = int(pairs.size());
+  const bool small = all_small(pairs);
+  if (small && count <= kParamRegions && param_shape(shape, true)) {
+    SmallPair entries[kParamRegions];
+    for (int i = 0; i < count; ++i)
+      entries[i] = make_small(pairs[i]);
+    err = launch_param(entries, count, uint32_t(chunks), 0, shape.ctas_per_sm, s);
+    if (!err)
+      set_last_kernel("batch_copy");
+    return err;
+  }
+  std::vector<SmallPair> entries;
+  if (small)
+    entries = small_table(pairs);
+  const void *from = small ? static_cast<const void *>(entries.data())
+                           : static_cast<const void *>(pairs.data());
+  const size_t bytes = pairs.size() * (small ? sizeof(SmallPair) : sizeof(CopyPair));
+  if (bytes > capacity) {
     cudaFree(table);
     table = nullptr;
     capacity = 0;
-    on_device.clear();
-    const size_t want = std::max<size_t>(pairs.size(), 64);
-    cudaError_t e = cudaMalloc(&table, want * sizeof(CopyPair));
+    cudaError_t e = cudaMalloc(&table, bytes);
     if (e != cudaSuccess)
       return cuda_error(e, "copy table allocation");
-    capacity = want;
+    capacity = bytes;
   }
-  // a loop that exchanges the same regions every step uploads its table once
-  const size_t bytes = pairs.size() * sizeof(CopyPair);
-  if (on_device.size() != pairs.size() ||
-      std::memcmp(on_device.data(), pairs.data(), bytes) != 0) {
-    on_device.clear();
-    cudaError_t e = cudaMemcpyAsync(table, pairs.data(), bytes,
-                                    cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess)
-      return cuda_error(e, "copy table upload");
-    on_device = pairs;
-    on_device_sig = sig;
-  }
-  return launch_table(table, int(pairs.size()), uint32_t(chunks), 0, shape, s);
+  cudaError_t e = cudaMemcpyAsync(table, from, bytes, cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess)
+    return cuda_error(e, "copy table upload");
+  return launch_table<CopyPair>(table, count, small, uint32_t(chunks), 0, shape, s);
 }
 
 } // namespace tempi
@@ -868,11 +1213,10 @@ int replan(tempi_batch *b, const Tuned &t) {
   int err;
   if (!bi.host_pairs.empty()) {
     chunks = apply_passes(bi.host_pairs, &t);
-    err = upload(bi.host_pairs, &bi.dev_pairs);
   } else {
     chunks = apply_passes(bi.host, &t);
-    err = upload(bi.host, &bi.dev);
   }
+  err = upload_table(bi);
   if (chunks > UINT32_MAX)
     return set_error(TEMPI_ERR_ARG, "batch too large");
   bi.total_chunks = uint32_t(chunks);
@@ -954,7 +1298,9 @@ extern "C" int tempi_batch_tune(tempi_batch *b, void *stream, int32_t reps) {
       Tuned t = best;
       t.shape.threads = th;
       t.shape.ctas_per_sm = cps;
-      if (cps > max_ctas(!bi.host_pairs.empty(), th, 0) ||
+      if (cps > max_ctas(!bi.host_pairs.empty() ? kind_of<CopyPair>(bi.small, 0)
+                                            : kind_of<BatchRegion>(bi.small, bi.unpack),
+                         th, 0) ||
           (th == best.shape.threads && cps == best.shape.ctas_per_sm))
         continue;
       err = replan(b, t);
@@ -1074,13 +1420,13 @@ static_assert(sizeof(StaticPiece<kFillPiece>) + 8 <= 32764,
 // entries [first, first + count) of the array from the piece, a 32-bit
 // word per thread; the host guarantees first + count <= kStaticBatchRegions
 // and count <= P
-template <int P>
+template <int P, typename Rec>
 __global__ void __launch_bounds__(256)
-    k_static_fill(const __grid_constant__ StaticPiece<P> piece, int first,
+    k_static_fill(const __grid_constant__ StaticPiece<P, Rec> piece, int first,
                   int count) {
-  constexpr int kWords = sizeof(BatchRegion) / 4;
+  constexpr int kWords = sizeof(Rec) / 4;
   const uint32_t *from = reinterpret_cast<const uint32_t *>(piece.r);
-  uint32_t *to = reinterpret_cast<uint32_t *>(g_static_regions + first);
+  uint32_t *to = reinterpret_cast<uint32_t *>(g_static_regions) + first * kWords;
   for (int w = threadIdx.x; w < count * kWords; w += blockDim.x)
     to[w] = from[w];
 }
@@ -1108,20 +1454,32 @@ static int static_table(BatchRegion **out) {
 }
 
 // launch k_static_fill for entries [first, first + count) of `piece`
-static int static_fill(const StaticPiece<kFillPiece> &piece, int first,
+template <typename Rec>
+static int static_fill(const StaticPiece<kFillPiece, Rec> &piece, int first,
                        int count, cudaStream_t s) {
-  if (count <= 32) { // a small table: a 5.4 KB parameter block
-    StaticPiece<32> small;
-    std::memcpy(small.r, piece.r, size_t(count) * sizeof(BatchRegion));
-    k_static_fill<32><<<1, 256, 0, s>>>(small, first, count);
+  if (count <= 32) { // a small table: a quarter of the parameter block
+    StaticPiece<32, Rec> few;
+    std::memcpy(few.r, piece.r, size_t(count) * sizeof(Rec));
+    k_static_fill<32, Rec><<<1, 256, 0, s>>>(few, first, count);
   } else {
-    k_static_fill<kFillPiece><<<1, 256, 0, s>>>(piece, first, count);
+    k_static_fill<kFillPiece, Rec><<<1, 256, 0, s>>>(piece, first, count);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return cuda_error(e, "static region table fill");
   counters().kernel_launches++;
   return TEMPI_OK;
+}
+
+// the same from full entries, compacted first when `small`
+static int static_fill(const StaticPiece<kFillPiece> &piece, int first,
+                       int count, bool small, cudaStream_t s) {
+  if (!small)
+    return static_fill<BatchRegion>(piece, first, count, s);
+  StaticPiece<kFillPiece, SmallRegion> compact;
+  for (int i = 0; i < count; ++i)
+    compact.r[i] = make_small(piece.r[i]);
+  return static_fill<SmallRegion>(compact, first, count, s);
 }
 
 extern "C" int tempi_batch_run_static(const tempi_region *regions, int32_t n,
@@ -1142,11 +1500,24 @@ extern "C" int tempi_batch_run_static(const tempi_region *regions, int32_t n,
   StaticPiece<kFillPiece> piece;
   int used = 0, filled = 0;
   uint64_t chunks = 0;
+  uint64_t compact = 0;
+  bool small = true; // every entry, once pass 0 is over
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1 && used <= kParamRegions) { // pass 0 left them all in piece
       if (used == 0)
         return TEMPI_OK;
-      err = launch_param(piece.r, used, uint32_t(chunks), unpack ? 1 : 0, 3, s);
+      if (small) {
+        SmallRegion few[kParamRegions];
+        chunks = 0;
+        for (int i = 0; i < used; ++i) {
+          piece.r[i].chunk_begin = uint32_t(chunks);
+          chunks += chunks_of(piece.r[i].g, piece.r[i].passes, true);
+          few[i] = make_small(piece.r[i]);
+        }
+        err = launch_param(few, used, uint32_t(chunks), unpack ? 1 : 0, 0, s);
+      } else {
+        err = launch_param(piece.r, used, uint32_t(chunks), unpack ? 1 : 0, 0, s);
+      }
       if (!err)
         set_last_kernel(unpack ? "batch_unpack_static" : "batch_pack_static");
       return err;
@@ -1168,20 +1539,24 @@ extern "C" int tempi_batch_run_static(const tempi_region *regions, int32_t n,
       br.strided = strided;
       br.packed = (char *)r.packed;
       br.passes = default_passes(region_class(br.g));
+      small = small && is_small(br); // settled by pass 0
       br.chunk_begin = uint32_t(chunks);
-      const uint64_t per = 32ull * lane_words_of(br.g.width) * br.passes;
-      chunks += (br.g.total_words + per - 1) / per;
+      chunks += chunks_of(br.g, br.passes, pass == 1 && small);
       if (chunks > UINT32_MAX)
         return set_error(TEMPI_ERR_ARG, "batch too large");
+      if (pass == 0) {
+        compact += chunks_of(br.g, br.passes, true);
+        small = small && compact <= UINT32_MAX;
+      }
       if (++filled == kFillPiece) {
-        if (pass == 1 && (err = static_fill(piece, used, filled, s)))
+        if (pass == 1 && (err = static_fill(piece, used, filled, small, s)))
           return err;
         used += filled;
         filled = 0;
       }
     }
     if (filled) { // a partial last piece (empty regions are never stored)
-      if (pass == 1 && (err = static_fill(piece, used, filled, s)))
+      if (pass == 1 && (err = static_fill(piece, used, filled, small, s)))
         return err;
       used += filled;
       filled = 0;
@@ -1189,7 +1564,8 @@ extern "C" int tempi_batch_run_static(const tempi_region *regions, int32_t n,
   }
   if (used == 0)
     return TEMPI_OK;
-  err = launch_table(table, used, uint32_t(chunks), unpack ? 1 : 0, Shape{}, s);
+  err = launch_table<BatchRegion>(table, used, small, uint32_t(chunks), unpack ? 1 : 0,
+                                  Shape{}, s);
   if (err)
     return err;
   set_last_kernel(unpack ? "batch_unpack_static" : "batch_pack_static");
@@ -1204,7 +1580,6 @@ extern "C" int tempi_batch_destroy(tempi_batch *b) {
   if (b->impl.graph)
     cudaGraphDestroy(b->impl.graph);
   cudaFree(b->impl.dev);
-  cudaFree(b->impl.dev_pairs);
   delete b;
   return TEMPI_OK;
 }

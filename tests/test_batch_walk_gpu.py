@@ -1,0 +1,137 @@
+"""The compact batch kernels step from word to word by adding to a word's
+digits instead of dividing its index: every way a step of 32 words can carry
+(row lengths and counts around 32, one word, one row), at every word width,
+with few regions (their table in the kernel's parameters) and with many (in
+device memory, its first chunks in shared memory or not)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tempi_b200 import _lib
+
+from . import helpers as H
+from .test_canon import desc_pack
+from .test_exchange_gpu import desc_unpack
+
+pytestmark = pytest.mark.gpu
+
+WORDS_PER_ROW = (1, 2, 3, 31, 32, 33, 65)
+COUNTS = ((), (2,), (33,), (1, 5), (3, 7), (31, 2), (32, 3), (70, 2))
+
+
+def layouts(width):
+    """Descriptors of `width`-byte words: every row length x every count."""
+    out = []
+    for wpr in WORDS_PER_ROW:
+        for counts in COUNTS:
+            inner, strides = wpr * width, []
+            for c in counts:
+                strides.append(inner + width * 3)
+                inner = c * strides[-1]
+            out.append(_lib.Desc.make(width * 2, inner + width * 2, wpr * width, list(counts),
+                                      strides))
+    return out
+
+
+def place(descs, width):
+    regs, typed, packed = [], 0, 0
+    for d in descs:
+        regs.append((typed, d, packed))
+        typed += d.extent + 64 // width * width
+        packed += d.size + 2 * width
+    return regs, typed + 64, packed + 64
+
+
+def launch(regs, tp, pp, unpack):
+    arr = (_lib.Region * len(regs))()
+    for k, (b, d, off) in enumerate(regs):
+        arr[k].origin, arr[k].packed = tp + b, pp + off
+        arr[k].desc, arr[k].incount = d, 1
+    h = ctypes.c_void_p()
+    _lib.check(_lib.tempi().tempi_batch_create(arr, len(regs), unpack, ctypes.byref(h)))
+    _lib.check(_lib.tempi().tempi_batch_launch(h, None))
+    return h
+
+
+@pytest.mark.parametrize("per_batch", [28, 10000])
+@pytest.mark.parametrize("width", [1, 2, 4, 8, 16])
+def test_every_carry(cuda, mpi_init, width, per_batch):
+    import torch
+
+    descs = layouts(width)
+    regs, nt, npk = place(descs, width)
+    typed_np, packed_np = H.splitmix_bytes(nt, width), H.splitmix_bytes(npk, 50 + width)
+    typed = torch.from_numpy(typed_np).cuda()
+    packed = torch.full((npk,), 0x5A, dtype=torch.uint8, device="cuda")
+    into = torch.full((nt,), 0xAA, dtype=torch.uint8, device="cuda")
+    source = torch.from_numpy(packed_np).cuda()
+    handles = []
+    for i in range(0, len(regs), per_batch):
+        part = regs[i: i + per_batch]
+        handles.append(launch(part, typed.data_ptr(), packed.data_ptr(), 0))
+        handles.append(launch(part, into.data_ptr(), source.data_ptr(), 1))
+    torch.cuda.synchronize()
+    for h in handles:
+        _lib.tempi().tempi_batch_destroy(h)
+    want, back = np.full(npk, 0x5A, np.uint8), np.full(nt, 0xAA, np.uint8)
+    for b, d, off in regs:
+        want[off: off + d.size] = desc_pack(d, typed_np[b:], 1)
+        desc_unpack(d, packed_np[off: off + d.size], back[b:], 1)
+    assert packed.cpu().numpy().tobytes() == want.tobytes()
+    assert into.cpu().numpy().tobytes() == back.tobytes()
+
+
+def test_more_regions_than_shared_memory_holds(cuda, mpi_init):
+    """9,000 regions: the search for a chunk's region reads the table."""
+    import torch
+
+    descs = [_lib.Desc.make(4 * (k % 3), 256, 4 * (k % 7 + 1), [k % 4 + 1], [44])
+             for k in range(9000)]
+    regs, nt, npk = place(descs, 4)
+    typed_np = H.splitmix_bytes(nt, 9)
+    typed = torch.from_numpy(typed_np).cuda()
+    packed = torch.full((npk,), 0x5A, dtype=torch.uint8, device="cuda")
+    h = launch(regs, typed.data_ptr(), packed.data_ptr(), 0)
+    torch.cuda.synchronize()
+    _lib.tempi().tempi_batch_destroy(h)
+    want = np.full(npk, 0x5A, np.uint8)
+    for b, d, off in regs:
+        want[off: off + d.size] = desc_pack(d, typed_np[b:], 1)
+    assert packed.cpu().numpy().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("width", [1, 4, 8, 16])
+def test_copy_between_walks(cuda, mpi_init, width):
+    """Copy pairs whose two sides step differently through the same words."""
+    import torch
+
+    sides = [d for d in layouts(width) if d.ndims]
+    pairs, ns, nd = [], 0, 0
+    for s in sides:
+        words = s.size // width
+        row = max(r for r in (1, 2, 5, 33) if words % r == 0)
+        d = _lib.Desc.make(width, words // row * (row + 1) * width + width, row * width,
+                           [words // row], [(row + 1) * width])
+        pairs.append((ns, s, nd, d))
+        ns += s.extent + 16 * width
+        nd += d.extent + 16 * width
+    src_np = H.splitmix_bytes(ns + 64, 3)
+    src = torch.from_numpy(src_np).cuda()
+    dst = torch.full((nd + 64,), 0xAA, dtype=torch.uint8, device="cuda")
+    for i in range(0, len(pairs), 30):
+        part = pairs[i: i + 30]
+        arr = (_lib.CopyRegion * len(part))()
+        for k, (sb, s, db, d) in enumerate(part):
+            arr[k].src_origin, arr[k].dst_origin = src.data_ptr() + sb, dst.data_ptr() + db
+            arr[k].src_desc, arr[k].dst_desc = s, d
+            arr[k].src_count = arr[k].dst_count = 1
+        h = ctypes.c_void_p()
+        _lib.check(_lib.tempi().tempi_batch_create_copy(arr, len(part), ctypes.byref(h)))
+        _lib.check(_lib.tempi().tempi_batch_launch(h, None))
+        torch.cuda.synchronize()
+        _lib.tempi().tempi_batch_destroy(h)
+    want = np.full(nd + 64, 0xAA, np.uint8)
+    for sb, s, db, d in pairs:
+        desc_unpack(d, desc_pack(s, src_np[sb:], 1), want[db:], 1)
+    assert dst.cpu().numpy().tobytes() == want.tobytes()
