@@ -135,3 +135,66 @@ def test_copy_between_walks(cuda, mpi_init, width):
     for sb, s, db, d in pairs:
         desc_unpack(d, desc_pack(s, src_np[sb:], 1), want[db:], 1)
     assert dst.cpu().numpy().tobytes() == want.tobytes()
+
+
+def test_dependent_launches_overlap_safely(cuda, mpi_init):
+    """Batches launched back to back on one stream, each reading what the one
+    before wrote: a kernel may start early but touches no buffer before the
+    kernels ahead of it have finished."""
+    import torch
+
+    from tempi_b200 import halo, mpi
+
+    g = halo.Grid((70, 45, 33), 2)
+    start = H.splitmix_bytes(g.nbytes, 77)
+    data = torch.from_numpy(start).cuda()
+    packed = torch.zeros(g.packed_bytes, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.Stream()
+    pack = halo.HaloBatch([g], [data.data_ptr()], [packed.data_ptr()])
+    fill = halo.HaloBatch([g], [data.data_ptr()], [packed.data_ptr()], unpack=True)
+    want = start.copy()
+    order = [(d, tuple(-x for x in d)) for d in halo.directions()]
+    descs = {}
+    for d, _ in order:
+        descs[d, False] = mpi.describe(g.send[d])[1]
+        descs[d, True] = mpi.describe(g.recv[d])[1]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for k in range(40):
+            pack.launch(stream.cuda_stream)
+            fill.launch(stream.cuda_stream)
+            data.add_(1)  # an ordinary kernel between overlapped ones
+    stream.synchronize()
+    for k in range(40):
+        bytes_of = {d: desc_pack(descs[d, False], want, 1) for d, _ in order}
+        for d, opposite in order:
+            desc_unpack(descs[opposite, True], bytes_of[d], want, 1)
+        last = np.concatenate([bytes_of[d] for d, _ in order])
+        want += np.uint8(1)
+    assert packed.cpu().numpy().tobytes() == last.tobytes()
+    assert data.cpu().numpy().tobytes() == want.tobytes()
+    # two batches straight after each other, many times: the second undoes
+    # nothing and reads only finished bytes
+    for k in range(50):
+        pack.launch(stream.cuda_stream)
+        fill.launch(stream.cuda_stream)
+    stream.synchronize()
+    bytes_of = {d: desc_pack(descs[d, False], want, 1) for d, _ in order}
+    for d, opposite in order:
+        desc_unpack(descs[opposite, True], bytes_of[d], want, 1)
+    assert data.cpu().numpy().tobytes() == want.tobytes()
+    # launches inside a capture become ordinary nodes
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        data.add_(3)
+        pack.launch(stream.cuda_stream)
+        fill.launch(stream.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    want += np.uint8(3)
+    bytes_of = {d: desc_pack(descs[d, False], want, 1) for d, _ in order}
+    for d, opposite in order:
+        desc_unpack(descs[opposite, True], bytes_of[d], want, 1)
+    assert data.cpu().numpy().tobytes() == want.tobytes()
+    pack.close()
+    fill.close()
