@@ -87,7 +87,9 @@ typedef struct tempi_desc {
    with bulk stores, else pulls 8 KB chunks in and scatters them by vector
    words.  Every staged launch needs a packed size that is a multiple
    of 16 and device memory on both sides; calls that do not qualify take the
-   automatic rules).  width: vector bytes for kernels 1, 2 and 4
+   automatic rules), 5 realign kernel (rows of 16 B or more at any alignment:
+   a thread per 16-B word of the destination; `unroll` = 1 or 4 words in
+   flight per thread).  width: vector bytes for kernels 1, 2 and 4
    (1,2,4,8,16; never above what the alignment proof allows).
    blocks_per_sm: resident blocks per SM the grid is sized for (kernel 4:
    1..8; the 16 KB-chunk kernels run one warp per block, one block per SM

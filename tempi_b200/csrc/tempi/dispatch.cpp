@@ -432,7 +432,7 @@ void remember_layout(const std::string &key, int choice) {
   g_layouts[key] = choice;
 }
 
-tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
+static tempi_config choose(TypeRecord &r, int64_t incount, bool src_host,
                            bool dst_host, bool unpack) {
   const Dispatch mode = env().dispatch;
   if (mode == Dispatch::HEURISTIC || mode == Dispatch::TABLE || g_measuring)
@@ -516,6 +516,15 @@ tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
   r.configs[key] = choice;
   remember_layout(lkey, choice);
   return choice < 0 ? tempi_config{} : kCandidates[choice];
+}
+
+tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
+                           bool dst_host, bool unpack) {
+  tempi_config c = choose(r, incount, src_host, dst_host, unpack);
+  // the exhaustive policy runs exactly what it measured
+  if (env().dispatch != Dispatch::EXHAUSTIVE)
+    c.reserved = kOwnChoice;
+  return c;
 }
 
 Method choose_method(TypeRecord &r, int count) {

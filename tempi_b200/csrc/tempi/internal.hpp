@@ -124,6 +124,11 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t strided_base,
                   uintptr_t packed_base, int max_width, Geometry *g,
                   bool *empty);
 
+// tempi_config::reserved of a configuration the dispatcher chose: the launch
+// may still take the realign kernel (pack.cu realign_wins), which is not among
+// the candidates the cost model scores.
+constexpr int32_t kOwnChoice = 0x7e91;
+
 // Launch one pack (unpack=false) or unpack on `stream`.  both_device: 1 when
 // the caller knows both buffers are device memory proper, 0 when it knows
 // they are not, -1 to ask the runtime (only the staged kernels need it).

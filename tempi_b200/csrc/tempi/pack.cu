@@ -24,6 +24,9 @@
 //    wide rows.
 //  * k_rows_shift: a group of lanes per row, 16-B words realigned by funnel
 //    shifts, for rows whose two sides disagree modulo 16.
+//  * k_realign: a thread per 16-B word of the destination, built from the two
+//    aligned source words that cover it: odd rows too short, too few or too
+//    long for the shift kernel's group of lanes per row, device memory only.
 //  * k_unpack_staged: 8 KB chunks of the packed stream move into shared
 //    memory by bulk asynchronous copies counted on mbarriers (bounded
 //    waits), and are scattered to the rows by plain vector stores.
@@ -276,6 +279,172 @@ __global__ void __launch_bounds__(256)
       shifted_row<L>(p, s, n, lane);
     else
       shifted_row<L>(s, p, n, lane);
+  }
+}
+
+// Word copy for rows whose two sides disagree modulo 16 (or whose lengths are
+// not a multiple of 16): every thread builds whole 16-byte words of the
+// destination from the two aligned 16-byte source words that cover each, four
+// words in flight.  Neighbouring lanes share source words, so the second load
+// of a lane is an L1 hit on its neighbour's first.
+//   pack    the destination words are those of the packed stream, aligned in
+//           memory, so all but the first and last are stored whole; a word
+//           that runs past its row's end takes the rest from the next row
+//           (rows of 16 B or more: it touches at most two);
+//   unpack  each row owns `slots` destination words, enough at any
+//           alignment; its partial end words are stored in pieces.
+// A source word is loaded only if it holds a byte of the row (unpack: of the
+// packed buffer).  Long streams are bound by DRAM: a 60 MB run at an odd
+// offset packs in 20 us beyond the call's fixed cost, 0.92 of the copy peak
+// (the word kernel, at a byte a thread: 44 us).
+constexpr int64_t kRealignMinRow = 16; // a packed word touches at most two rows
+constexpr int kRealignThreads = 256;
+
+struct Realign {
+  FastDiv div;    // pack: by the row's bytes; unpack: by `slots`
+  uint32_t words; // pack: 16-byte words of the packed stream; unpack: slots
+  uint32_t bytes; // packed bytes
+};
+
+// the two aligned words covering [base + off, base + off + 16), each only if
+// it holds one of the bytes [base, base + n); returns the shift in bytes
+__device__ __forceinline__ uint32_t load_pair(const char *base, int off, int n,
+                                              uint4 *a, uint4 *b) {
+  const char *p = base + off;
+  const uint32_t m = uint32_t(reinterpret_cast<uintptr_t>(p) & 15);
+  const uint4 *q = reinterpret_cast<const uint4 *>(p - m);
+  const int lo = off - int(m); // of the first word, relative to base
+  *a = lo > -16 && lo < n ? __ldg(q) : make_uint4(0, 0, 0, 0);
+  *b = m && lo > -32 && lo + 16 < n ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
+  return m;
+}
+
+// bytes [0, k) of x, the others of y
+__device__ __forceinline__ uint4 join(const uint4 &x, const uint4 &y, int k) {
+  auto one = [&](uint32_t u, uint32_t v, int kk) {
+    const uint32_t keep = kk <= 0 ? 0u : kk >= 4 ? 0xffffffffu
+                                                 : (1u << (8 * kk)) - 1;
+    return (u & keep) | (v & ~keep);
+  };
+  return make_uint4(one(x.x, y.x, k), one(x.y, y.y, k - 4),
+                    one(x.z, y.z, k - 8), one(x.w, y.w, k - 12));
+}
+
+// bytes [m, m + 16) of the 32 bytes a, b: two rounds of selects and a funnel
+// shift, without branches (m differs from row to row within a warp)
+__device__ __forceinline__ uint4 cut16(const uint4 &a, const uint4 &b, uint32_t m) {
+  const bool two = m & 8, one = m & 4;
+  const uint32_t y0 = two ? a.z : a.x, y1 = two ? a.w : a.y,
+                 y2 = two ? b.x : a.z, y3 = two ? b.y : a.w,
+                 y4 = two ? b.z : b.x, y5 = two ? b.w : b.y;
+  const uint32_t x0 = one ? y1 : y0, x1 = one ? y2 : y1, x2 = one ? y3 : y2,
+                 x3 = one ? y4 : y3, x4 = one ? y5 : y4;
+  const uint32_t sh = (m & 3) * 8;
+  return make_uint4(__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh),
+                    __funnelshift_r(x2, x3, sh), __funnelshift_r(x3, x4, sh));
+}
+
+// Bytes [a, b) of v to w + a (w 16-B aligned, 0 <= a < b <= 16, one of a = 0
+// and b = 16) in at most four aligned pieces, without a loop.
+__device__ __forceinline__ void store_end(char *w, const uint4 &v, uint32_t a,
+                                          uint32_t b) {
+  if (b == 16) { // the head of a row: ascending pieces
+    if (a & 1) {
+      w[a] = char(word32(v, a >> 2) >> ((a & 3) * 8));
+      ++a;
+    }
+    if (a & 2) {
+      *reinterpret_cast<uint16_t *>(w + a) = uint16_t(word32(v, a >> 2) >> ((a & 3) * 8));
+      a += 2;
+    }
+    if (a & 4) {
+      *reinterpret_cast<uint32_t *>(w + a) = word32(v, a >> 2);
+      a += 4;
+    }
+    if (a & 8)
+      *reinterpret_cast<uint2 *>(w + 8) = make_uint2(v.z, v.w);
+  } else { // the tail: descending pieces
+    if (b & 8)
+      *reinterpret_cast<uint2 *>(w) = make_uint2(v.x, v.y);
+    if (b & 4)
+      *reinterpret_cast<uint32_t *>(w + (b & 8)) = b & 8 ? v.z : v.x;
+    const uint32_t x = word32(v, b >> 2);
+    if (b & 2)
+      *reinterpret_cast<uint16_t *>(w + (b & 12)) = uint16_t(x);
+    if (b & 1)
+      w[b & 14] = char(x >> ((b & 2) * 8));
+  }
+}
+
+template <int U, int ND, bool UNPACK>
+__global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 6)
+    k_realign(char *__restrict__ strided, char *__restrict__ packed,
+              const __grid_constant__ Geometry g,
+              const __grid_constant__ Realign r) {
+  const int n = int(g.block), total = int(r.bytes);
+  const uint32_t tile = blockDim.x * U;
+  const uint32_t a0 = uint32_t(reinterpret_cast<uintptr_t>(packed) & 15);
+  for (uint32_t t0 = blockIdx.x * tile + threadIdx.x; t0 < r.words;
+       t0 += gridDim.x * tile) {
+    uint4 a[U], b[U];
+    uint32_t m[U];
+    int at[U]; // pack: column of the word's first byte; unpack: the same,
+               // relative to the row
+    char *to[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t t = t0 + u * blockDim.x;
+      if (t >= r.words) {
+        at[u] = 0x7fffffff;
+        continue;
+      }
+      if (!UNPACK) {
+        const int p = int(16 * t - a0);
+        const uint32_t row = fastdiv(p < 0 ? 0u : uint32_t(p), r.div);
+        at[u] = p - int(row) * n;
+        m[u] = load_pair(strided + row_offset<ND>(row, g), at[u], n, &a[u], &b[u]);
+      } else {
+        const uint32_t row = fastdiv(t, r.div), j = t - row * r.div.d;
+        char *d = strided + row_offset<ND>(row, g);
+        const uint32_t lo = uint32_t(reinterpret_cast<uintptr_t>(d) & 15);
+        at[u] = int(16 * j) - int(lo);
+        if (at[u] >= n) {
+          at[u] = 0x7fffffff;
+          continue;
+        }
+        to[u] = d + at[u];
+        m[u] = load_pair(packed, int(row) * n + at[u], total, &a[u], &b[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (at[u] == 0x7fffffff)
+        continue;
+      uint4 v = cut16(a[u], b[u], m[u]);
+      if (!UNPACK) {
+        const int p = int(16 * (t0 + u * blockDim.x) - a0);
+        const int k = n - at[u]; // bytes this row still has
+        if (k < 16 && p + k < total) {
+          const uint32_t row = fastdiv(p < 0 ? 0u : uint32_t(p), r.div) + 1;
+          uint4 c, d;
+          const uint32_t mm =
+              load_pair(strided + row_offset<ND>(row, g), -k, n, &c, &d);
+          v = join(v, cut16(c, d, mm), k);
+        }
+        char *w = packed + p;
+        if (p >= 0 && p + 16 <= total)
+          *reinterpret_cast<uint4 *>(w) = v;
+        else
+          store_part(w, v, p < 0 ? uint32_t(-p) : 0u,
+                     p + 16 <= total ? 16u : uint32_t(total - p)); // once a pack
+      } else {
+        if (at[u] >= 0 && at[u] + 16 <= n)
+          *reinterpret_cast<uint4 *>(to[u]) = v;
+        else
+          store_end(to[u], v, at[u] < 0 ? uint32_t(-at[u]) : 0u,
+                    at[u] + 16 <= n ? 16u : uint32_t(n - at[u]));
+      }
+    }
   }
 }
 
@@ -795,6 +964,18 @@ template <bool UNPACK> KernelFn pick(int kernel, uint32_t width, uint32_t nd) {
   }
 }
 
+using RealignFn = void (*)(char *, char *, Geometry, Realign);
+template <int U, bool UNPACK> RealignFn pick_realign(uint32_t nd) {
+  switch (nd) {
+  case 0: return k_realign<U, 0, UNPACK>;
+  case 1: return k_realign<U, 1, UNPACK>;
+  case 2: return k_realign<U, 2, UNPACK>;
+  case 3: return k_realign<U, 3, UNPACK>;
+  case 4: return k_realign<U, 4, UNPACK>;
+  default: return k_realign<U, 5, UNPACK>;
+  }
+}
+
 static const char *kernel_name(int kernel, uint32_t width, bool unpack) {
   static char names[4][2][33][32];
   static std::once_flag once;
@@ -927,11 +1108,95 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t sbase,
   return TEMPI_OK;
 }
 
+// Whether the realign kernel takes a launch whose kernel the library chooses
+// (device memory on both sides).  Measured on B200 by synchronised calls over
+// 590 random layouts whose rows are not 16-byte words, against the kernel the
+// cost model or the fixed rules pick (its time / the realign kernel's, mean):
+//  * rows of 8 KiB and more in 32 MiB and more (contiguous runs among them):
+//    1.06 for 4- and 8-byte words, 1.5 for narrower ones (a 60 MB run at an
+//    odd offset 54 -> 30 us);
+//  * odd rows (1- and 2-byte words) of 4 KiB and more, too few to give every
+//    SM 16 warps a row each, from 2 MB: 1.07 to 1.3;
+//  * short odd rows: packs below 128 B from 2 MB 1.08 to 1.5, unpacks of 64
+//    to 255 B from 4 MB 1.02 to 1.26;
+//  * unpacks of rows below 2 KiB in 64 MB and more: 1.05 to 1.09 (3-D floats,
+//    262,144 rows of 256 B: 61 -> 57 us).
+// Between these, odd rows of 256 B to 4 KiB run 3 to 9 % faster with a group
+// of lanes per row (the shift kernel), and 4- and 8-byte words of rows the
+// L2 holds with the word kernels, whose few instructions cost less latency.
+static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack, int sms) {
+  if (g.width >= 16 || g.block < kRealignMinRow)
+    return false;
+  constexpr uint64_t MB = 1000000;
+  if (g.block >= 8192 && bytes >= (uint64_t(32) << 20))
+    return true;
+  if (unpack && g.block < 2048 && g.block >= 64 && bytes >= 64 * MB)
+    return true;
+  if (g.width > 2)
+    return false;
+  if (g.block >= 4096)
+    return g.rows < uint32_t(16 * sms) && bytes >= 2 * MB;
+  return unpack ? g.block >= 64 && g.block < 256 && bytes >= 4 * MB
+                : g.block < 128 && bytes >= 2 * MB;
+}
+
+static int launch_realign(const Geometry &g, char *strided, char *packed,
+                          bool unpack, const tempi_config *cfg,
+                          cudaStream_t stream) {
+  Realign r{};
+  r.bytes = g.rows * uint32_t(g.block);
+  if (unpack) {
+    // destination words a row can touch, whatever its alignment
+    const uint32_t slots = uint32_t((g.block + 30) / 16);
+    r.div = make_fastdiv(slots);
+    r.words = g.rows * slots;
+  } else {
+    const uint32_t a0 = uint32_t(reinterpret_cast<uintptr_t>(packed) & 15);
+    r.div = make_fastdiv(uint32_t(g.block));
+    r.words = uint32_t((uint64_t(a0) + r.bytes + 15) / 16);
+  }
+  // one word a thread for small objects and short rows (less code to fetch,
+  // more warps), four for long streams (10 % faster from 32 MB on)
+  const int asked = cfg && cfg->kernel == 5 ? cfg->unroll : 0;
+  const uint32_t words = asked == 1 || asked == 4 ? uint32_t(asked)
+                         : r.bytes >= 8000000u && g.block >= 4096 ? 4u
+                                                                  : 1u;
+  const uint32_t per = uint32_t(kRealignThreads) * words;
+  uint32_t blocks = (r.words + per - 1) / per;
+  if (cfg && cfg->kernel == 5 && cfg->blocks_per_sm > 0)
+    blocks = uint32_t(std::min<int64_t>(
+        blocks, int64_t(num_sms()) * cfg->blocks_per_sm));
+  const RealignFn fn = words == 1 ? (unpack ? pick_realign<1, true>(g.nd)
+                                            : pick_realign<1, false>(g.nd))
+                                  : (unpack ? pick_realign<4, true>(g.nd)
+                                            : pick_realign<4, false>(g.nd));
+  fn<<<blocks, kRealignThreads, 0, stream>>>(strided, packed, g, r);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess)
+    return cuda_error(e, "realign kernel launch");
+  counters().kernel_launches++;
+  set_last_kernel(unpack ? "realign_unpack" : "realign_pack");
+  return TEMPI_OK;
+}
+
 int launch_geometry(const Geometry &g, const char *strided, char *packed,
                     bool unpack, const tempi_config *cfg, cudaStream_t stream,
                     int both_device) {
   const int sms = num_sms();
   int kernel = cfg ? cfg->kernel : 0;
+  if (kernel == 5 && g.block >= kRealignMinRow)
+    return launch_realign(g, const_cast<char *>(strided), packed, unpack, cfg,
+                          stream);
+  // the library's own choice of kernel: by the fixed rules (none asked for) or
+  // by the dispatcher
+  const bool own = kernel < 1 || kernel > 5 || cfg->reserved == kOwnChoice;
+  if (own && realign_wins(g, uint64_t(g.rows) * uint64_t(g.block), unpack, sms)) {
+    if (both_device < 0)
+      both_device = classify(strided).is_device && classify(packed).is_device;
+    if (both_device)
+      return launch_realign(g, const_cast<char *>(strided), packed, unpack, cfg,
+                            stream);
+  }
   // the staged kernels (4), where their bulk copies are allowed: unpack
   // needs a 16-B aligned packed base and a packed size that is a multiple of
   // 16 bytes; pack needs every row piece 16-B aligned on both sides (width
