@@ -17,18 +17,19 @@
 
 namespace tempi {
 
-// the kernel configurations the model scores (outputs 0..9)
+// the kernel configurations the model scores (outputs 0..9), measured and
+// launched as the dispatcher's own choice (kOwnChoice)
 const tempi_config kCandidates[kNumConfigs] = {
-    {1, 0, 256, 0, 0, 0},  // word kernel, 256 threads
-    {1, 0, 512, 0, 0, 0},  // word kernel, 512 threads
-    {1, 0, 128, 0, 0, 0},  // word kernel, 128 threads
-    {2, 0, 256, 0, 0, 0},  // row kernel (warp per row)
-    {3, 0, 256, 4, 0, 0},  // shift kernel, 4 lanes per row
-    {3, 0, 256, 8, 0, 0},  // shift kernel, 8 lanes per row
-    {3, 0, 256, 16, 0, 0}, // shift kernel, 16 lanes per row
-    {3, 0, 256, 32, 0, 0}, // shift kernel, 32 lanes per row
-    {4, 0, 256, 0, 3, 0},  // staged kernel, 3 CTAs per SM
-    {4, 0, 256, 0, 8, 0},  // staged kernel, 8 CTAs per SM
+    {1, 0, 256, 0, 0, kOwnChoice},  // word kernel, 256 threads
+    {1, 0, 512, 0, 0, kOwnChoice},  // word kernel, 512 threads
+    {1, 0, 128, 0, 0, kOwnChoice},  // word kernel, 128 threads
+    {2, 0, 256, 0, 0, kOwnChoice},  // row kernel (warp per row)
+    {3, 0, 256, 4, 0, kOwnChoice},  // shift kernel, 4 lanes per row
+    {3, 0, 256, 8, 0, kOwnChoice},  // shift kernel, 8 lanes per row
+    {3, 0, 256, 16, 0, kOwnChoice}, // shift kernel, 16 lanes per row
+    {3, 0, 256, 32, 0, kOwnChoice}, // shift kernel, 32 lanes per row
+    {4, 0, 256, 0, 3, kOwnChoice},  // staged kernel, 3 CTAs per SM
+    {4, 0, 256, 0, 8, kOwnChoice},  // staged kernel, 8 CTAs per SM
 };
 
 namespace {
@@ -432,7 +433,7 @@ void remember_layout(const std::string &key, int choice) {
   g_layouts[key] = choice;
 }
 
-static tempi_config choose(TypeRecord &r, int64_t incount, bool src_host,
+tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
                            bool dst_host, bool unpack) {
   const Dispatch mode = env().dispatch;
   if (mode == Dispatch::HEURISTIC || mode == Dispatch::TABLE || g_measuring)
@@ -516,15 +517,6 @@ static tempi_config choose(TypeRecord &r, int64_t incount, bool src_host,
   r.configs[key] = choice;
   remember_layout(lkey, choice);
   return choice < 0 ? tempi_config{} : kCandidates[choice];
-}
-
-tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
-                           bool dst_host, bool unpack) {
-  tempi_config c = choose(r, incount, src_host, dst_host, unpack);
-  // the exhaustive policy runs exactly what it measured
-  if (env().dispatch != Dispatch::EXHAUSTIVE)
-    c.reserved = kOwnChoice;
-  return c;
 }
 
 Method choose_method(TypeRecord &r, int count) {
