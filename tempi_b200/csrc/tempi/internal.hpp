@@ -130,8 +130,10 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t strided_base,
 constexpr int32_t kOwnChoice = 0x7e91;
 
 // Launch one pack (unpack=false) or unpack on `stream`.  both_device: 1 when
-// the caller knows both buffers are device memory proper, 0 when it knows
-// they are not, -1 to ask the runtime (only the staged kernels need it).
+// the caller knows both buffers are device memory proper, kBothHost when it
+// knows both are pinned host memory, 0 when it knows they are neither, -1 to
+// ask the runtime where it matters.
+constexpr int kBothHost = 2;
 int launch_geometry(const Geometry &g, const char *strided_base, char *packed,
                     bool unpack, const tempi_config *cfg, cudaStream_t stream,
                     int both_device = -1);

@@ -54,6 +54,11 @@ HostLink use_host_link(const PtrInfo &a, const PtrInfo &b, const tempi_desc &d,
   return unpack && host_rows(d, count, rows) ? HostLink::ROWS : HostLink::NONE;
 }
 
+// launch_geometry's both_device
+int where(const PtrInfo &a, const PtrInfo &b) {
+  return a.is_device && b.is_device ? 1 : a.is_host && b.is_host ? kBothHost : 0;
+}
+
 // A contiguous device buffer goes through host staging under
 // TEMPI_CONTIGUOUS_STAGED always, under TEMPI_CONTIGUOUS_AUTO when the
 // measured tables say staging is faster (reference types_init and
@@ -178,7 +183,7 @@ int MPI_Pack(const void *inbuf, int incount, MPI_Datatype datatype,
         choose_config(*r, incount, in.is_host, out.is_host, false);
     e = pack_known(&r->desc, in.device_ptr, incount,
                    static_cast<char *>(out.device_ptr) + *position, &cfg, s,
-                   in.is_device && out.is_device ? 1 : 0);
+                   where(in, out));
   }
   if (!e) {
     cudaError_t ce = cudaStreamSynchronize(s);
@@ -236,7 +241,7 @@ int MPI_Unpack(const void *inbuf, int insize, int *position, void *outbuf,
     e = unpack_known(&r->desc,
                      static_cast<const char *>(in.device_ptr) + *position,
                      outcount, out.device_ptr, &cfg, s,
-                     in.is_device && out.is_device ? 1 : 0);
+                     where(in, out));
   }
   if (!e) {
     cudaError_t ce = cudaStreamSynchronize(s);

@@ -1179,6 +1179,10 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
   return TEMPI_OK;
 }
 
+// Smallest object whose buffers are looked up, when the caller does not know
+// where they are, for the host-link grid (smaller ones fit it anyway).
+constexpr uint64_t kLinkMinBytes = uint64_t(512) << 10;
+
 int launch_geometry(const Geometry &g, const char *strided, char *packed,
                     bool unpack, const tempi_config *cfg, cudaStream_t stream,
                     int both_device) {
@@ -1193,7 +1197,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   if (own && realign_wins(g, uint64_t(g.rows) * uint64_t(g.block), unpack, sms)) {
     if (both_device < 0)
       both_device = classify(strided).is_device && classify(packed).is_device;
-    if (both_device)
+    if (both_device == 1)
       return launch_realign(g, const_cast<char *>(strided), packed, unpack, cfg,
                             stream);
   }
@@ -1268,6 +1272,10 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
     else
       kernel = 1;
   }
+  const bool both_host =
+      both_device == kBothHost ||
+      (both_device < 0 && bytes >= kLinkMinBytes && classify(strided).is_host &&
+       classify(packed).is_host);
   // rows per group of lanes for the shift kernel
   uint32_t lanes = 32;
   if (kernel == 3) {
@@ -1292,6 +1300,23 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
     need = (int64_t(g.total_words) + int64_t(threads) * kUnroll - 1) /
            (int64_t(threads) * kUnroll);
   int64_t blocks = std::min<int64_t>(need, int64_t(sms) * bps);
+  // Both sides in host memory: few enough loads in flight that the first
+  // stores go out while most loads are still to be issued.  With a full grid
+  // every read of a 4 MiB object is queued on the link before the first write,
+  // and the two directions run one after the other: 1-KiB rows 159 us at 1184
+  // CTAs, 143 at 148, 122 at 8 to 32 (16-B words, 256 threads); 256-B rows of
+  // 4-B words 182 at 1184, 151 at 96 to 148, 177 at 16.  So the grid holds
+  // about 640 KB in flight, counting only the lanes that a row keeps busy
+  // (64-B rows are bound by the number of requests and keep the full grid).
+  if (both_host) {
+    const int64_t n = g.block;
+    const int64_t flight =
+        kernel == 1   ? int64_t(threads) * kUnroll * g.width
+        : kernel == 2 ? threads / 32 * std::min<int64_t>(n, 32 * kUnroll * g.width)
+                      : threads / int(lanes) *
+                            std::min<int64_t>(n, lanes * kShiftWords * 16);
+    blocks = std::min<int64_t>(blocks, (int64_t(640) << 10) / flight);
+  }
   blocks = std::max<int64_t>(blocks, 1);
   const uint32_t sel = kernel == 3 ? lanes : g.width;
   KernelFn fn = unpack ? pick<true>(kernel, sel, g.nd)
