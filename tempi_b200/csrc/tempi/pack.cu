@@ -294,7 +294,12 @@ __global__ void __launch_bounds__(256)
 //   unpack  each row owns `slots` destination words, enough at any
 //           alignment; its partial end words are stored in pieces.
 // A source word is loaded only if it holds a byte of the row (unpack: of the
-// packed buffer).  Long streams are bound by DRAM: a 60 MB run at an odd
+// packed buffer).  An unpack of rows whose ends cut 32-byte sectors, into
+// buffers that the L2 does not hold, asks for the cut lines along with the
+// packed words: a line that a row fills only in part has to be merged with
+// memory when it leaves the L2, and done then that costs twice the fetch
+// (262,144 rows of 64 B in one line each: 25 us plain, 19 with the fetch, 12.6
+// when the rows are sector-aligned).  Long streams are bound by DRAM: a 60 MB run at an odd
 // offset packs in 20 us beyond the call's fixed cost, 0.92 of the copy peak
 // (the word kernel, at a byte a thread: 44 us).
 constexpr int64_t kRealignMinRow = 16; // a packed word touches at most two rows
@@ -304,7 +309,12 @@ struct Realign {
   FastDiv div;    // pack: by the row's bytes; unpack: by `slots`
   uint32_t words; // pack: 16-byte words of the packed stream; unpack: slots
   uint32_t bytes; // packed bytes
+  uint32_t edges; // unpack: fetch the lines that a row's ends cut
 };
+
+__device__ __forceinline__ void fetch_line(const char *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 
 // the two aligned words covering [base + off, base + off + 16), each only if
 // it holds one of the bytes [base, base + n); returns the shift in bytes
@@ -413,6 +423,8 @@ __global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 6)
           continue;
         }
         to[u] = d + at[u];
+        if (r.edges && (at[u] <= 0 || at[u] + 16 >= n))
+          fetch_line(at[u] < 0 ? d : to[u]);
         m[u] = load_pair(packed, int(row) * n + at[u], total, &a[u], &b[u]);
       }
     }
@@ -1119,18 +1131,19 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t sbase,
 //    SM 16 warps a row each, from 2 MB: 1.07 to 1.3;
 //  * short odd rows: packs below 128 B from 2 MB 1.08 to 1.5, unpacks of 64
 //    to 255 B from 4 MB 1.02 to 1.26;
-//  * unpacks of rows below 2 KiB in 64 MB and more: 1.05 to 1.09 (3-D floats,
-//    262,144 rows of 256 B: 61 -> 57 us).
+//  * unpacks of 64-B to 2-KiB rows that cut sectors, in more than the L2 keeps
+//    (cuts_sectors below): 1.02 to 1.4.
 // Between these, odd rows of 256 B to 4 KiB run 3 to 9 % faster with a group
 // of lanes per row (the shift kernel), and 4- and 8-byte words of rows the
 // L2 holds with the word kernels, whose few instructions cost less latency.
-static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack, int sms) {
+static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack,
+                         bool cut, int sms) {
+  if (cut)
+    return true;
   if (g.width >= 16 || g.block < kRealignMinRow)
     return false;
   constexpr uint64_t MB = 1000000;
   if (g.block >= 8192 && bytes >= (uint64_t(32) << 20))
-    return true;
-  if (unpack && g.block < 2048 && g.block >= 64 && bytes >= 64 * MB)
     return true;
   if (g.width > 2)
     return false;
@@ -1140,11 +1153,31 @@ static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack, int sms
                 : g.block < 128 && bytes >= 2 * MB;
 }
 
+// Whether an unpack's rows leave partial sectors in lines that the L2 will not
+// hold until they are filled: rows of 64 B to 2 KiB with an end off a 32-byte
+// boundary, and packed bytes plus touched lines of 48 MB or more (the 126 MB
+// L2 works in two halves, and a program rarely unpacks into one buffer alone).
+// Measured with the realign kernel against the plain choice, synchronised:
+// 64-B rows 37 -> 26 us in one line, 37 -> 33 across two; 200-B rows 43 -> 35;
+// 256-B rows 48 -> 36; 512-B 31 -> 30; 1000-B 28 -> 27.  Below 42 MB the lines
+// are in the L2 and the word kernels are up to 8 % faster; rows below 64 B,
+// with no full sector of their own, gain nothing or lose (32 B: 14.6 -> 18.5).
+static bool cuts_sectors(const Geometry &g, const char *strided) {
+  if (g.block < 64 || g.block >= 2048 ||
+      uint64_t(g.rows) * uint64_t(2 * g.block + 128) < 48000000)
+    return false;
+  uint64_t bits = uint64_t(g.block) | reinterpret_cast<uintptr_t>(strided);
+  for (uint32_t k = 0; k < g.nd; ++k)
+    bits |= uint64_t(g.strides[k]);
+  return bits & 31;
+}
+
 static int launch_realign(const Geometry &g, char *strided, char *packed,
-                          bool unpack, const tempi_config *cfg,
+                          bool unpack, bool cut, const tempi_config *cfg,
                           cudaStream_t stream) {
   Realign r{};
   r.bytes = g.rows * uint32_t(g.block);
+  r.edges = cut;
   if (unpack) {
     // destination words a row can touch, whatever its alignment
     const uint32_t slots = uint32_t((g.block + 30) / 16);
@@ -1156,11 +1189,13 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
     r.words = uint32_t((uint64_t(a0) + r.bytes + 15) / 16);
   }
   // one word a thread for small objects and short rows (less code to fetch,
-  // more warps), four for long streams (10 % faster from 32 MB on)
+  // more warps), four for long streams (10 % faster from 32 MB on) and for
+  // longer rows with cut ends (4 % from 400 B on)
   const int asked = cfg && cfg->kernel == 5 ? cfg->unroll : 0;
   const uint32_t words = asked == 1 || asked == 4 ? uint32_t(asked)
-                         : r.bytes >= 8000000u && g.block >= 4096 ? 4u
-                                                                  : 1u;
+                         : r.bytes >= 8000000u && g.block >= (cut ? 384 : 4096)
+                             ? 4u
+                             : 1u;
   const uint32_t per = uint32_t(kRealignThreads) * words;
   uint32_t blocks = (r.words + per - 1) / per;
   if (cfg && cfg->kernel == 5 && cfg->blocks_per_sm > 0)
@@ -1188,18 +1223,20 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
                     int both_device) {
   const int sms = num_sms();
   int kernel = cfg ? cfg->kernel : 0;
+  const bool cut = unpack && cuts_sectors(g, strided);
   if (kernel == 5 && g.block >= kRealignMinRow)
-    return launch_realign(g, const_cast<char *>(strided), packed, unpack, cfg,
-                          stream);
+    return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
+                          cfg, stream);
   // the library's own choice of kernel: by the fixed rules (none asked for) or
   // by the dispatcher
   const bool own = kernel < 1 || kernel > 5 || cfg->reserved == kOwnChoice;
-  if (own && realign_wins(g, uint64_t(g.rows) * uint64_t(g.block), unpack, sms)) {
+  if (own && realign_wins(g, uint64_t(g.rows) * uint64_t(g.block), unpack, cut,
+                          sms)) {
     if (both_device < 0)
       both_device = classify(strided).is_device && classify(packed).is_device;
     if (both_device == 1)
-      return launch_realign(g, const_cast<char *>(strided), packed, unpack, cfg,
-                            stream);
+      return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
+                            cfg, stream);
   }
   // the staged kernels (4), where their bulk copies are allowed: unpack
   // needs a 16-B aligned packed base and a packed size that is a multiple of

@@ -83,7 +83,12 @@ def test_dimensions(cuda, mpi_init, nd):
     (1, 256, [16_000], [259], (None, None)),
     (1, 4097, [2300], [4101], ("realign", "realign")),     # too few rows for a warp each
     (1, 4097, [2400], [4101], (None, None)),
-    (4, 260, [250_000], [264], (None, "realign")),         # 64 MB of short rows
+    (4, 260, [76_000], [264], (None, "realign")),          # rows that cut sectors, 49 MB
+    (4, 260, [70_000], [264], (None, None)),               # ... 45 MB
+    (16, 64, [190_000], [96], (None, "realign")),          # 16-byte words too
+    (32, 64, [190_000], [96], (None, None)),               # whole sectors
+    (16, 48, [250_000], [96], (None, None)),
+    (16, 2048, [12_000], [2080], (None, None)),
 ])
 def test_automatic_choice(cuda, mpi_init, start, block, counts, strides, kernels):
     sms = _sms()
