@@ -1128,7 +1128,8 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t sbase,
 //    1.06 for 4- and 8-byte words, 1.5 for narrower ones (a 60 MB run at an
 //    odd offset 54 -> 30 us);
 //  * odd rows (1- and 2-byte words) of 4 KiB and more, too few to give every
-//    SM 16 warps a row each, from 2 MB: 1.07 to 1.3;
+//    SM 16 warps a row each, from 2 MB: 1.07 to 1.3 (4-byte words of 8 KiB
+//    rows from 16 MB: 1.2, where the pick is a kernel by rows);
 //  * short odd rows: packs below 128 B from 2 MB 1.08 to 1.5, unpacks of 64
 //    to 255 B from 4 MB 1.02 to 1.26;
 //  * unpacks of 64-B to 2-KiB rows that cut sectors, in more than the L2 keeps
@@ -1145,6 +1146,8 @@ static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack,
   constexpr uint64_t MB = 1000000;
   if (g.block >= 8192 && bytes >= (uint64_t(32) << 20))
     return true;
+  if (g.width == 4 && g.nd > 0 && g.block >= 8192 && g.rows < uint32_t(16 * sms))
+    return bytes >= 16 * MB;
   if (g.width > 2)
     return false;
   if (g.block >= 4096)
@@ -1155,16 +1158,21 @@ static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack,
 
 // Whether an unpack's rows leave partial sectors in lines that the L2 will not
 // hold until they are filled: rows of 64 B to 2 KiB with an end off a 32-byte
-// boundary, and packed bytes plus touched lines of 48 MB or more (the 126 MB
-// L2 works in two halves, and a program rarely unpacks into one buffer alone).
-// Measured with the realign kernel against the plain choice, synchronised:
-// 64-B rows 37 -> 26 us in one line, 37 -> 33 across two; 200-B rows 43 -> 35;
-// 256-B rows 48 -> 36; 512-B 31 -> 30; 1000-B 28 -> 27.  Below 42 MB the lines
-// are in the L2 and the word kernels are up to 8 % faster; rows below 64 B,
-// with no full sector of their own, gain nothing or lose (32 B: 14.6 -> 18.5).
+// boundary, and packed bytes plus touched lines of 60 MB or more, or 48 MB for
+// 1- and 2-byte words, whose other kernels are slower (the 126 MB L2 works in
+// two halves, and a program rarely unpacks into one buffer alone).  Measured
+// with the realign kernel against the best other choice, synchronised, three
+// buffer sets in turn: 64-B rows 37 -> 26 us in one line, 37 -> 33 across two;
+// 200-B rows 43 -> 35; 256-B rows 48 -> 36; over 75 random layouts above the
+// line 1.0 to 1.3 for 4- to 16-byte words (0.92 to 0.97 in three with hardly
+// any gap between rows), 1.1 to 1.7 for narrower ones.  Below it the lines are
+// in the L2 and the word and row kernels are up to 13 % faster; rows below
+// 64 B, with no full sector of their own, gain nothing or lose (32 B: 14.6 ->
+// 18.5 us).
 static bool cuts_sectors(const Geometry &g, const char *strided) {
   if (g.block < 64 || g.block >= 2048 ||
-      uint64_t(g.rows) * uint64_t(2 * g.block + 128) < 48000000)
+      uint64_t(g.rows) * uint64_t(2 * g.block + 128) <
+          (g.width <= 2 ? 48000000u : 60000000u))
     return false;
   uint64_t bits = uint64_t(g.block) | reinterpret_cast<uintptr_t>(strided);
   for (uint32_t k = 0; k < g.nd; ++k)
@@ -1190,10 +1198,10 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
   }
   // one word a thread for small objects and short rows (less code to fetch,
   // more warps), four for long streams (10 % faster from 32 MB on) and for
-  // longer rows with cut ends (4 % from 400 B on)
+  // longer rows with cut ends (up to 10 % from 256 B on)
   const int asked = cfg && cfg->kernel == 5 ? cfg->unroll : 0;
   const uint32_t words = asked == 1 || asked == 4 ? uint32_t(asked)
-                         : r.bytes >= 8000000u && g.block >= (cut ? 384 : 4096)
+                         : r.bytes >= 8000000u && g.block >= (cut ? 256 : 4096)
                              ? 4u
                              : 1u;
   const uint32_t per = uint32_t(kRealignThreads) * words;

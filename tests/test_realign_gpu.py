@@ -83,10 +83,13 @@ def test_dimensions(cuda, mpi_init, nd):
     (1, 256, [16_000], [259], (None, None)),
     (1, 4097, [2300], [4101], ("realign", "realign")),     # too few rows for a warp each
     (1, 4097, [2400], [4101], (None, None)),
-    (4, 260, [76_000], [264], (None, "realign")),          # rows that cut sectors, 49 MB
-    (4, 260, [70_000], [264], (None, None)),               # ... 45 MB
-    (16, 64, [190_000], [96], (None, "realign")),          # 16-byte words too
-    (32, 64, [190_000], [96], (None, None)),               # whole sectors
+    (4, 260, [93_000], [264], (None, "realign")),          # rows that cut sectors, 60.3 MB
+    (4, 260, [92_000], [264], (None, None)),               # ... 59.6 MB
+    (2, 262, [74_000], [266], (None, "realign")),          # ... 48.2 MB of 2-byte words
+    (16, 64, [240_000], [96], (None, "realign")),          # 16-byte words too
+    (32, 64, [240_000], [96], (None, None)),               # whole sectors
+    (4, 8196, [2300], [8212], ("realign", "realign")),     # long rows, too few of them
+    (4, 8196, [2400], [8212], (None, None)),
     (16, 48, [250_000], [96], (None, None)),
     (16, 2048, [12_000], [2080], (None, None)),
 ])
