@@ -18,16 +18,18 @@
 // Two sets of kernels do this.  Batches whose regions all have at most two
 // strided dimensions (every region of a grid) run the compact ones
 // (k_batch_small, k_batch_copy_small and their _param forms): 64-byte
-// entries, words reached by stepping their digits instead of dividing, 64
-// registers, launches that overlap the kernel before them (see
-// wait_for_previous).  What bounds them is the rate of scattered lines for the x faces
-// (about 41 G lines/s measured by a one-load gather) and, for small halos,
-// the launch itself.  Measured against the other set on B200, launches back to
-// back over rotating buffers, pack / unpack / exchange in us: 8 mixed grids
-// (208 regions, 16.8 MB) 24.0 / 17.6 / 28.8 before, 13.5 / 14.2 / 16.7 now;
-// 320 x 300 x 310 doubles radius 3 12.4 / 12.5 / 17.5 before, 10.5 / 8.6 /
-// 10.6 now.  The others (k_batch, k_batch_copy) divide every word's index
-// over any number of dimensions, at 80 registers.
+// entries, words reached by stepping their digits instead of dividing, one
+// code path for every width at 64 registers, and launches that overlap the
+// kernel before them (wait_for_previous).  What bounds them is the rate of
+// scattered lines of the x faces (about 41 G lines/s by a one-load gather) and,
+// for small halos, the launch.  Measured on B200, launches back to back over
+// rotating buffers, pack / unpack / exchange in us: 8 mixed grids (208
+// regions, 16.8 MB, whose lines take 9.8) 24.0 / 17.6 / 28.8 by the other
+// set, 10.5 / 10.9 / 14.4 by these; the 256^3 halo 8.0 / 7.8 / 8.5 and 4.3 /
+// 3.9 / 5.9; 320 x 300 x 310 doubles radius 3 12.4 / 12.5 / 17.5 and 7.0 /
+// 6.5 / 8.8.  A 256^3 pack alone on the GPU: 19.5 and 14.4 us a call.  The
+// other kernels (k_batch, k_batch_copy) divide every word's index over any
+// number of dimensions, at 80 registers.
 //
 // The passes of each region class (width x words per row) and the launch
 // shape of a batch (threads per CTA, CTAs per SM) come from defaults or from
@@ -111,23 +113,31 @@ struct Side {
 };
 
 // What the kernels read for a region or pair of at most two strided
-// dimensions: 64 and 104 bytes instead of 168 and 288, so a halo's 26 regions
-// take 2 KB of kernel parameters and one entry two sectors.
-struct SmallRegion {
+// dimensions: 64 and 112 bytes instead of 168 and 288, so a halo's 26 regions
+// take 2 KB of kernel parameters.  A warp loads the first 64 bytes of its
+// entry at once (four 16-byte loads, one round trip), a pair's destination
+// side behind its data loads.
+struct alignas(16) SmallRegion {
   Side s;
   char *packed;
   uint32_t total_words;
   uint32_t chunk_begin;
 };
 
-struct SmallPair {
-  Side s, d; // s.passes and s.lwidth hold for both
+struct alignas(16) SmallPair {
+  Side s; // its passes and lwidth hold for both sides
+  uint64_t spare;
   uint32_t total_words;
   uint32_t chunk_begin;
+  Side d;
 };
 static_assert(sizeof(Side) == 48 && sizeof(SmallRegion) == 64 &&
-                  sizeof(SmallPair) == 104,
-              "record sizes are documented");
+                  sizeof(SmallPair) == 112 && offsetof(SmallPair, d) == 64 &&
+                  offsetof(SmallPair, total_words) ==
+                      offsetof(SmallRegion, total_words) &&
+                  offsetof(SmallPair, chunk_begin) ==
+                      offsetof(SmallRegion, chunk_begin),
+              "entries start with 64 bytes of one layout");
 
 Side make_side(const char *base, const Geometry &g, uint32_t passes) {
   Side s{};
@@ -155,8 +165,8 @@ SmallRegion make_small(const BatchRegion &r) {
           r.chunk_begin};
 }
 SmallPair make_small(const CopyPair &r) {
-  return {make_side(r.src, r.gs, r.passes), make_side(r.dst, r.gd, r.passes),
-          r.gs.total_words, r.chunk_begin};
+  return {make_side(r.src, r.gs, r.passes), 0, r.gs.total_words, r.chunk_begin,
+          make_side(r.dst, r.gd, r.passes)};
 }
 
 template <int W> struct BWord;
@@ -416,60 +426,115 @@ struct Walk {
   }
 };
 
-// One pass of a warp over U x 32 words of a region: words w, w + 32, ... with
-// `left` > 0 words (signed) from w to the region's end.  U loads are in
-// flight per lane; offsets are walked, never held.  Loads bypass the L1: a
-// kernel may have started before the previous one wrote what it reads.
-template <int W, int U, bool UNPACK>
-__device__ __forceinline__ void move_words(const SmallRegion &r, uint32_t w,
-                                           int left) {
-  using T = typename BWord<W>::T;
-  char *strided = r.s.base;
-  T *packed = reinterpret_cast<T *>(r.packed) + w;
-  Walk at(w, r.s);
-  T v[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    if (32 * u < left)
-      v[u] = __ldcg(UNPACK ? packed + 32 * u
-                           : reinterpret_cast<const T *>(strided + at.off));
-    if (!UNPACK)
-      at.next();
+// The words of a lane's pass, whatever their width: U loads in flight, then U
+// stores.  The width is switched on around the loads and again around the
+// stores, and the offsets are computed outside: the code of a pass exists
+// once, not once a width (five copies of it, whose common arithmetic the
+// compiler hoists out of them, spill at 64 registers).  `at(u)` is the address
+// of word u, `left` the words from word 0 to the region's end (32 apart).
+// Loads bypass the L1: a kernel may have started before the previous one wrote
+// what it reads.
+template <int U, typename At>
+__device__ __forceinline__ void load_words(uint4 (&v)[U], uint32_t lwidth,
+                                           int left, At at) {
+#define TEMPI_EACH(...)                                                        \
+  _Pragma("unroll") for (int u = 0; u < U; ++u) if (32 * u < left) {           \
+    const char *p = at(u);                                                     \
+    __VA_ARGS__                                                                \
+  }                                                                            \
+  break;
+  switch (lwidth) {
+  case 4: TEMPI_EACH(v[u] = __ldcg(reinterpret_cast<const uint4 *>(p));)
+  case 3: TEMPI_EACH(const uint2 t = __ldcg(reinterpret_cast<const uint2 *>(p));
+                     v[u].x = t.x; v[u].y = t.y;)
+  case 2: TEMPI_EACH(v[u].x = __ldcg(reinterpret_cast<const uint32_t *>(p));)
+  case 1: TEMPI_EACH(v[u].x = __ldcg(reinterpret_cast<const uint16_t *>(p));)
+  default: TEMPI_EACH(v[u].x = __ldcg(reinterpret_cast<const uint8_t *>(p));)
   }
+}
+template <int U, typename At>
+__device__ __forceinline__ void store_words(const uint4 (&v)[U],
+                                            uint32_t lwidth, int left, At at) {
+  switch (lwidth) {
+  case 4: TEMPI_EACH(*reinterpret_cast<uint4 *>(const_cast<char *>(p)) = v[u];)
+  case 3: TEMPI_EACH(*reinterpret_cast<uint2 *>(const_cast<char *>(p)) =
+                         make_uint2(v[u].x, v[u].y);)
+  case 2: TEMPI_EACH(*reinterpret_cast<uint32_t *>(const_cast<char *>(p)) = v[u].x;)
+  case 1: TEMPI_EACH(*reinterpret_cast<uint16_t *>(const_cast<char *>(p)) =
+                         uint16_t(v[u].x);)
+  default: TEMPI_EACH(*const_cast<char *>(p) = char(v[u].x);)
+  }
+#undef TEMPI_EACH
+}
+
+// the offsets of the pass's words on a strided side
+template <int U> struct Offsets {
+  int64_t off[U];
+  __device__ __forceinline__ Offsets(uint32_t w, const Side &s) {
+    Walk at(w, s);
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    if (32 * u < left)
-      *(UNPACK ? reinterpret_cast<T *>(strided + at.off) : packed + 32 * u) = v[u];
-    if (UNPACK)
-      at.next();
+    for (int u = 0; u < U; ++u) {
+      off[u] = at.off;
+      if (u + 1 < U)
+        at.next();
+    }
+  }
+};
+
+// N 16-byte loads of a table entry, all in flight together
+template <int N, typename To>
+__device__ __forceinline__ To load_entry(const void *from) {
+  static_assert(sizeof(To) == 16 * N, "whole 16-byte words");
+  union Both {
+    uint4 q[N];
+    To to;
+    __device__ Both() {}
+  } u;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    u.q[i] = static_cast<const uint4 *>(from)[i];
+  return u.to;
+}
+
+// one pass of a warp over words w, w + 32, ... of a region
+template <bool UNPACK>
+__device__ __forceinline__ void move_words(const SmallRegion &r,
+                                           const SmallRegion *, uint32_t w,
+                                           int left) {
+  constexpr int U = kSmallWords;
+  const uint32_t lw = r.s.lwidth;
+  char *strided = r.s.base, *packed = r.packed + (uint64_t(w) << lw);
+  uint4 v[U];
+  auto in_packed = [&](int u) { return packed + (32u * u << lw); };
+  if (!UNPACK) {
+    const Offsets<U> o(w, r.s);
+    load_words<U>(v, lw, left, [&](int u) { return strided + o.off[u]; });
+    store_words<U>(v, lw, left, in_packed);
+  } else {
+    load_words<U>(v, lw, left, in_packed);
+    const Offsets<U> o(w, r.s);
+    store_words<U>(v, lw, left, [&](int u) { return strided + o.off[u]; });
   }
 }
 
-// one pass over a copy pair: the loads at the source side first, then the
-// stores at the destination side
-template <int W, int U, bool UNPACK>
-__device__ __forceinline__ void move_words(const SmallPair &r, uint32_t w,
+// and of a copy pair, `r` its first 64 bytes: the destination side is read and
+// its offsets are computed behind the data loads
+template <bool UNPACK>
+__device__ __forceinline__ void move_words(const SmallRegion &r,
+                                           const SmallPair *entry, uint32_t w,
                                            int left) {
-  using T = typename BWord<W>::T;
-  T v[U];
+  constexpr int U = kSmallWords;
+  const uint32_t lw = r.s.lwidth;
+  uint4 v[U];
   {
     const char *src = r.s.base;
-    Walk at(w, r.s);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (32 * u < left)
-        v[u] = __ldcg(reinterpret_cast<const T *>(src + at.off));
-      at.next();
-    }
+    const Offsets<U> o(w, r.s);
+    load_words<U>(v, lw, left, [&](int u) { return src + o.off[u]; });
   }
-  char *dst = r.d.base;
-  Walk at(w, r.d);
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    if (32 * u < left)
-      *reinterpret_cast<T *>(dst + at.off) = v[u];
-    at.next();
-  }
+  const Side d = load_entry<3, Side>(&entry->d);
+  char *dst = d.base;
+  const Offsets<U> o(w, d);
+  store_words<U>(v, lw, left, [&](int u) { return dst + o.off[u]; });
 }
 
 // Programmatic dependent launch.  A batch kernel lets the next kernel of its
@@ -478,8 +543,9 @@ __device__ __forceinline__ void move_words(const SmallPair &r, uint32_t w,
 // touches a buffer: launch latency and the reading of the table overlap the
 // kernel before.  Both are no-ops where a neighbour was launched without the
 // attribute.  Measured back to back on B200, per launch: a 64^3 grid (bound by
-// the launch) 6.2 us without, 2.6 us with; the 256^3 halo 7.3 and 4.5 us; 8
-// mixed grids 13.5 and 11.2 us.
+// the launch) 6.2 us without, 2.6 us with, 2.2 us with the first chunk's entry
+// looked up before the wait too; the 256^3 halo 7.3, 4.5 and 4.3 us; 8 mixed
+// grids 13.5, 11.2 and 10.5 us.
 __device__ __forceinline__ void let_next_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -502,32 +568,35 @@ __device__ __forceinline__ void small_chunks(const Rec *tab, int n,
       s_begin[i] = tab[i].chunk_begin;
     __syncthreads();
   }
-  wait_for_previous();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  int at = 0;
+  SmallRegion r; // the entry of chunk c
+  auto look_up = [&] {
+    at = staged ? find_region([&](int i) { return s_begin[i]; }, n, c, lane)
+                : find_region([&](int i) { return tab[i].chunk_begin; }, n, c, lane);
+    r = load_entry<4, SmallRegion>(tab + at);
+  };
+  // the first chunk's entry is at hand when the kernels before have finished
+  if (c < total_chunks)
+    look_up();
+  wait_for_previous();
 #pragma unroll 1
-  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       c < total_chunks; c += nwarps) {
-    const int at =
-        staged ? find_region([&](int i) { return s_begin[i]; }, n, c, lane)
-               : find_region([&](int i) { return tab[i].chunk_begin; }, n, c, lane);
-    const uint32_t lw = tab[at].s.lwidth, passes = tab[at].s.passes;
+  while (c < total_chunks) {
+    const uint32_t passes = r.s.passes;
     constexpr uint32_t per = 32 * kSmallWords;
-    uint32_t w = (c - tab[at].chunk_begin) * passes * per + lane;
+    uint32_t w = (c - r.chunk_begin) * passes * per + lane;
 #pragma unroll 1
     for (uint32_t p = 0; p < passes; ++p, w += per) {
-      const Rec &r = tab[at];
       const int left = int(r.total_words - w);
       if (left <= 0)
         break;
-      switch (lw) {
-      case 4: move_words<16, kSmallWords, UNPACK>(r, w, left); break;
-      case 3: move_words<8, kSmallWords, UNPACK>(r, w, left); break;
-      case 2: move_words<4, kSmallWords, UNPACK>(r, w, left); break;
-      case 1: move_words<2, kSmallWords, UNPACK>(r, w, left); break;
-      default: move_words<1, kSmallWords, UNPACK>(r, w, left); break;
-      }
+      move_words<UNPACK>(r, tab + at, w, left);
     }
+    c += nwarps;
+    if (c < total_chunks)
+      look_up();
   }
 }
 
@@ -818,8 +887,6 @@ struct BatchImpl {
   std::vector<CopyPair> host_pairs; // a copy batch
   void *dev = nullptr; // the table: compact entries when `small`
   bool small = false;
-  std::vector<SmallRegion> host_small; // the table of a small pack batch
-  std::vector<SmallPair> host_pairs_small; // and of a small copy batch
   uint32_t total_chunks = 0;
   int unpack = 0;
   Shape shape;
@@ -885,16 +952,12 @@ static int upload(const std::vector<Rec> &recs, void **dev) {
 static int upload_table(BatchImpl &bi) {
   if (!bi.host_pairs.empty()) {
     bi.small = all_small(bi.host_pairs);
-    if (!bi.small)
-      return upload(bi.host_pairs, &bi.dev);
-    bi.host_pairs_small = small_table(bi.host_pairs);
-    return upload(bi.host_pairs_small, &bi.dev);
+    return bi.small ? upload(small_table(bi.host_pairs), &bi.dev)
+                    : upload(bi.host_pairs, &bi.dev);
   }
   bi.small = all_small(bi.host);
-  if (!bi.small)
-    return upload(bi.host, &bi.dev);
-  bi.host_small = small_table(bi.host);
-  return upload(bi.host_small, &bi.dev);
+  return bi.small ? upload(small_table(bi.host), &bi.dev)
+                  : upload(bi.host, &bi.dev);
 }
 
 extern "C" int tempi_batch_create(const tempi_region *regions, int32_t n,
@@ -943,9 +1006,9 @@ template <int P, typename Rec = BatchRegion> struct StaticPiece {
 
 // A batch of up to kParamRegions regions in one launch with its table in the
 // kernel's parameters (2 KB of compact entries, or 5.4 KB for more than two
-// strided dimensions), read there in place.  Used by the allocation-free
-// entry point (neither a fill kernel nor the fixed array is involved) and by
-// small batches at the default launch shape.
+// strided dimensions), for calls that bring their regions with them: the
+// allocation-free entry point (neither a fill kernel nor the fixed array is
+// involved) and the interposed MPI_Neighbor_alltoallw (no upload).
 constexpr int kParamRegions = 32;
 
 template <int P>
@@ -957,12 +1020,21 @@ __global__ void __launch_bounds__(256, 3)
   batch_chunks<256>(piece.r, nregions, total_chunks, unpack);
 }
 
+// The parameter block as ordinary memory: read through the constant cache,
+// the entries that an SM's warps share miss one after another (a 256^3
+// exchange alone on the GPU 19.3 us a call that way, 18.2 this way).
+template <typename Rec>
+__device__ __forceinline__ const Rec *in_memory(const Rec *param) {
+  asm volatile("" : "+l"(param));
+  return param;
+}
+
 template <int P, bool UNPACK>
 __global__ void __launch_bounds__(256, kSmallThreadsPerSm / 256)
     k_batch_param_small(const __grid_constant__ StaticPiece<P, SmallRegion> piece,
                         int nregions, uint32_t total_chunks) {
   __shared__ uint32_t s_begin[P];
-  small_chunks<UNPACK>(piece.r, nregions, total_chunks, 1, s_begin);
+  small_chunks<UNPACK>(in_memory(piece.r), nregions, total_chunks, 1, s_begin);
 }
 
 template <int P>
@@ -970,7 +1042,7 @@ __global__ void __launch_bounds__(256, kSmallThreadsPerSm / 256)
     k_batch_copy_param(const __grid_constant__ StaticPiece<P, SmallPair> piece,
                        int npairs, uint32_t total_chunks) {
   __shared__ uint32_t s_begin[P];
-  small_chunks<false>(piece.r, npairs, total_chunks, 1, s_begin);
+  small_chunks<false>(in_memory(piece.r), npairs, total_chunks, 1, s_begin);
 }
 
 // k_batch_param(_small) over the `n` <= kParamRegions entries of `table`
@@ -1006,43 +1078,20 @@ static int launch_param(const Rec *table, int n, uint32_t total_chunks,
   return TEMPI_OK;
 }
 
-// whether a launch shape is one that the parameter kernels can take
-static bool param_shape(const Shape &shape, bool small) {
-  return (shape.threads == 0 || shape.threads == 256) &&
-         (small || shape.ctas_per_sm <= 3);
-}
-
-// `direct`: a launch of its own (tempi_batch_launch).  There a small table at
-// a 256-thread shape rides in the kernel's parameters instead of being read
-// from device memory by every CTA (measured on the 256^3 halo: 11.3 against
-// 12.0-12.3 us by events, 7.3-7.6 against 7.6-7.9 us in-kernel).  Graph
-// captures and the tuner's timings keep the table in device memory: a
-// replayed kernel node with 5.4 KB of parameters measured 1-2 us slower.
+// `direct`: a launch of its own (tempi_batch_launch), which may overlap the
+// kernel before it; graph captures and the tuner's timings are plain.  The
+// table stays in device memory for all of them: with the same entries in the
+// kernel's parameters a 256^3 pack alone on the GPU took 17.2 us a call
+// against 14.4 (a parameter block is new memory at every launch, the table is
+// in the L2).
 static int batch_launch(tempi_batch *b, cudaStream_t s, bool direct) {
   BatchImpl &bi = b->impl;
-  const bool copy = !bi.host_pairs.empty();
-  const int n = int(copy ? bi.host_pairs.size() : bi.host.size());
-  if (direct && n > 0 && n <= kParamRegions && bi.total_chunks > 0 &&
-      param_shape(bi.shape, bi.small) && (bi.small || !copy)) {
-    const int per_sm = bi.shape.ctas_per_sm;
-    const int err =
-        copy ? launch_param(bi.host_pairs_small.data(), n, bi.total_chunks, 0,
-                            per_sm, s)
-        : bi.small ? launch_param(bi.host_small.data(), n, bi.total_chunks,
-                                  bi.unpack, per_sm, s)
-                   : launch_param(bi.host.data(), n, bi.total_chunks,
-                                  bi.unpack, per_sm, s);
-    if (!err)
-      set_last_kernel(copy        ? "batch_copy"
-                      : bi.unpack ? "batch_unpack"
-                                  : "batch_pack");
-    return err;
-  }
-  if (copy)
-    return launch_table<CopyPair>(bi.dev, n, bi.small, bi.total_chunks, 0,
-                                  bi.shape, s, direct);
-  return launch_table<BatchRegion>(bi.dev, n, bi.small, bi.total_chunks,
-                                   bi.unpack, bi.shape, s, direct);
+  if (!bi.host_pairs.empty())
+    return launch_table<CopyPair>(bi.dev, int(bi.host_pairs.size()), bi.small,
+                                  bi.total_chunks, 0, bi.shape, s, direct);
+  return launch_table<BatchRegion>(bi.dev, int(bi.host.size()), bi.small,
+                                   bi.total_chunks, bi.unpack, bi.shape, s,
+                                   direct);
 }
 
 // Copy pairs for `regions`, each at the default passes of its class; empty
@@ -1152,7 +1201,8 @@ int copy_batch_run(const tempi_copy_region *regions, int32_t n,
   }
   const int count = int(pairs.size());
   const bool small = all_small(pairs);
-  if (small && count <= kParamRegions && param_shape(shape, true)) {
+  if (small && count <= kParamRegions &&
+      (shape.threads == 0 || shape.threads == 256)) {
     SmallPair entries[kParamRegions];
     for (int i = 0; i < count; ++i)
       entries[i] = make_small(pairs[i]);
