@@ -261,6 +261,14 @@ TypeRecord *find_type(MPI_Datatype t) {
   return it == g_cache.end() ? nullptr : &it->second;
 }
 
+void find_types(const MPI_Datatype *t, int n, const TypeRecord **out) {
+  std::lock_guard<std::mutex> l(g_mu);
+  for (int i = 0; i < n; ++i) {
+    auto it = g_cache.find(t[i]);
+    out[i] = it == g_cache.end() ? nullptr : &it->second;
+  }
+}
+
 TypeRecord *commit_type(MPI_Datatype t) {
   {
     std::lock_guard<std::mutex> l(g_mu);
@@ -270,6 +278,13 @@ TypeRecord *commit_type(MPI_Datatype t) {
   }
   TypeRecord r;
   r.packable = canonicalize(t, &r.desc) == TEMPI_OK;
+  r.has_unit = r.packable && r.desc.size > 0;
+  for (int k = 0; k < 5 && r.has_unit; ++k) {
+    bool empty = false;
+    r.has_unit = make_geometry(&r.desc, 1, 0, 0, 1 << k, &r.unit[k], &empty) ==
+                     TEMPI_OK &&
+                 !empty;
+  }
   std::lock_guard<std::mutex> l(g_mu);
   auto res = g_cache.emplace(t, std::move(r));
   if (res.second)

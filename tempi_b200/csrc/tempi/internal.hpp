@@ -158,10 +158,19 @@ bool staged_channel(cudaStream_t stream);
 // failure word.
 bool staged_failed();
 
-// The copy batch's kernel (tempi_batch_create_copy) for one call, with its
-// pair table in a grow-only device buffer; launches on `s`, which the caller
-// synchronises before calling again.
-int copy_batch_run(const tempi_copy_region *regions, int32_t n,
-                   cudaStream_t s);
+// One edge of an exchange: `src_count` objects of a committed type at
+// `src_origin` into `dst_count` objects of another at `dst_origin`, equal in
+// packed bytes.
+struct TypeRecord;
+struct CopyEdge {
+  const TypeRecord *src_type, *dst_type;
+  const char *src_origin;
+  char *dst_origin;
+  int src_count, dst_count;
+};
+
+// The copy batch's kernel (tempi_batch_create_copy) for one call; launches on
+// `s`, which the caller synchronises before calling again.
+int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s);
 
 } // namespace tempi

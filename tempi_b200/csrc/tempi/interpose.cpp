@@ -18,6 +18,7 @@
 #include "runtime.hpp"
 #include "sender.hpp"
 
+#include <algorithm>
 #include <vector>
 
 namespace tempi {
@@ -383,33 +384,32 @@ int MPI_Neighbor_alltoallw(const void *sendbuf, const int sendcounts[],
   const PtrInfo ps = classify(sendbuf), pr = classify(recvbuf);
   bool any_described = false, fusable = indeg == outdeg && ps.device_accessible &&
                                         pr.device_accessible;
-  std::vector<tempi_copy_region> regs;
+  const int types = std::max(indeg, outdeg);
+  std::vector<const TypeRecord *> ts(size_t(types) + 1), tr(size_t(types) + 1);
+  find_types(sendtypes, outdeg, ts.data());
+  find_types(recvtypes, std::min(indeg, outdeg), tr.data());
+  std::vector<CopyEdge> edges;
+  edges.reserve(size_t(outdeg));
   for (int k = 0; k < outdeg; ++k) {
-    const TypeRecord *ts = find_type(sendtypes[k]);
-    const TypeRecord *tr = k < indeg ? find_type(recvtypes[k]) : nullptr;
-    const bool ds = ts && ts->packable, dr = tr && tr->packable;
+    const bool ds = ts[k] && ts[k]->packable, dr = tr[k] && tr[k]->packable;
     any_described = any_described || ds || dr;
     if (!fusable)
       continue;
     if (dests[k] != me || sources[k] != me || !ds || !dr ||
         sendcounts[k] < 0 || recvcounts[k] < 0 ||
-        int64_t(sendcounts[k]) * ts->desc.size !=
-            int64_t(recvcounts[k]) * tr->desc.size) {
+        int64_t(sendcounts[k]) * ts[k]->desc.size !=
+            int64_t(recvcounts[k]) * tr[k]->desc.size) {
       fusable = false;
       continue;
     }
-    tempi_copy_region c{};
-    c.src_origin = static_cast<const char *>(ps.device_ptr) + sdispls[k];
-    c.dst_origin = static_cast<char *>(pr.device_ptr) + rdispls[k];
-    c.src_desc = ts->desc;
-    c.dst_desc = tr->desc;
-    c.src_count = sendcounts[k];
-    c.dst_count = recvcounts[k];
-    regs.push_back(c);
+    edges.push_back({ts[k], tr[k],
+                     static_cast<const char *>(ps.device_ptr) + sdispls[k],
+                     static_cast<char *>(pr.device_ptr) + rdispls[k],
+                     sendcounts[k], recvcounts[k]});
   }
   if (fusable) {
     cudaStream_t s = pack_stream();
-    int e = copy_batch_run(regs.data(), int32_t(regs.size()), s);
+    int e = copy_batch_run(edges.data(), int(edges.size()), s);
     if (!e) {
       cudaError_t ce = cudaStreamSynchronize(s);
       if (ce != cudaSuccess)

@@ -62,6 +62,11 @@ int canonicalize(MPI_Datatype t, tempi_desc *out);
 struct TypeRecord {
   tempi_desc desc{};
   bool packable = false; // desc describes the type and a kernel handles it
+  // The geometries of one object at widths 1, 2, 4, 8 and 16 (no wider than
+  // the layout itself allows), settled at commit: calls with many regions
+  // (MPI_Neighbor_alltoallw) take the one that their pointers allow.
+  Geometry unit[5];
+  bool has_unit = false; // false: nothing to copy, or more than a launch takes
   // method chosen per packed byte count (reference SendRecvND's
   // modelChoiceCache_, sender.cpp:259-277)
   std::unordered_map<int64_t, Method> methods;
@@ -73,6 +78,8 @@ struct TypeRecord {
 // Returns nullptr when the type is unknown.  The pointer stays valid until
 // the type is released.
 TypeRecord *find_type(MPI_Datatype t);
+// `n` look-ups under one lock
+void find_types(const MPI_Datatype *t, int n, const TypeRecord **out);
 TypeRecord *commit_type(MPI_Datatype t);
 void release_type(MPI_Datatype t);
 

@@ -198,3 +198,58 @@ def test_dependent_launches_overlap_safely(cuda, mpi_init):
     assert data.cpu().numpy().tobytes() == want.tobytes()
     pack.close()
     fill.close()
+
+
+@pytest.mark.parametrize("edges", [3, 32, 33])
+@pytest.mark.parametrize("counts", [(1,), (1, 2), (1, 0, 3)])
+@pytest.mark.parametrize("offset", [0, 1, 4, 8])
+def test_exchange_of_committed_types(cuda, mpi_init, edges, counts, offset):
+    """MPI_Neighbor_alltoallw over self-edges, single objects (whose geometries
+    come from the commit) and several, at displacements that narrow the words,
+    among one, two and three strided dimensions, up to and past the number of
+    edges that fit the kernel's parameters."""
+    import torch
+
+    from tempi_b200 import mpi
+
+    def commit(shape):
+        block, c, s = shape
+        inner, t = block, mpi.Type_contiguous(block, mpi.BYTE)
+        for n, gap in zip(c, s):
+            t = mpi.Type_create_hvector(n, 1, inner + gap, t)
+            inner = (n - 1) * (inner + gap) + inner
+        t = mpi.Type_create_resized(t, 0, inner + 16 - inner % 16)
+        assert mpi.Type_commit(t) == 0
+        return t
+
+    kinds = [(48, (4,), (16,)), (16, (6, 2), (32, 16)), (24, (2, 2, 2), (8, 8, 8)), (192, (), ())]
+    types = [commit(k) for k in kinds]
+    descs = [mpi.describe(t)[1] for t in types]
+    assert len({d.size for d in descs}) == 1
+    sends = [k % 4 for k in range(edges)]
+    recvs = [(k + k // 4 + 1) % 4 for k in range(edges)]
+    n = [counts[k % len(counts)] for k in range(edges)]
+    at, sd, rd = 0, [], []
+    for k in range(edges):
+        sd.append(at + (offset if k % 3 else 0))
+        rd.append(at + 16)
+        at += 3 * 1024 + 64
+    src_np = H.splitmix_bytes(at + 64, edges)
+    src = torch.from_numpy(src_np).cuda()
+    dst = torch.full((at + 64,), 0xAA, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    err, comm = mpi.Dist_graph_create_adjacent([0] * edges, [0] * edges)
+    assert err == 0
+    before = _lib.counter("neighbor_fused")
+    for _ in range(2):
+        assert mpi.Neighbor_alltoallw(
+            src.data_ptr(), n, sd, [types[k] for k in sends], dst.data_ptr(), n, rd,
+            [types[k] for k in recvs], comm) == 0, _lib.last_error()
+    assert _lib.counter("neighbor_fused") == before + 2
+    want = np.full(at + 64, 0xAA, np.uint8)
+    for k in range(edges):
+        if n[k]:
+            got = desc_pack(descs[sends[k]], src_np[sd[k]:], n[k])
+            desc_unpack(descs[recvs[k]], got, want[rd[k]:], n[k])
+    assert dst.cpu().numpy().tobytes() == want.tobytes()
+    mpi.Comm_free(comm)
