@@ -271,7 +271,7 @@ int MPI_Send(const void *buf, int count, MPI_Datatype datatype, int dest,
   TypeRecord *r = p.device_accessible ? find_type(datatype) : nullptr;
   if (r && r->packable && r->desc.ndims >= 1 && count > 0) {
     Method m = choose_method(*r, count);
-    return send_strided(*r, m, p.device_ptr, count, dest, tag, comm);
+    return send_strided(*r, m, p, count, dest, tag, comm);
   }
   if (contiguous_staged(r, p, count)) {
     return send_contiguous_staged(buf, count, datatype,
@@ -293,7 +293,7 @@ int MPI_Recv(void *buf, int count, MPI_Datatype datatype, int source, int tag,
   TypeRecord *r = p.device_accessible ? find_type(datatype) : nullptr;
   if (r && r->packable && r->desc.ndims >= 1 && count > 0) {
     Method m = choose_method(*r, count);
-    return recv_strided(*r, m, p.device_ptr, count, source, tag, comm, status);
+    return recv_strided(*r, m, p, count, source, tag, comm, status);
   }
   if (contiguous_staged(r, p, count)) {
     return recv_contiguous_staged(buf, count, datatype,
@@ -316,7 +316,7 @@ int MPI_Isend(const void *buf, int count, MPI_Datatype datatype, int dest,
   int err;
   if (r && r->packable && r->desc.ndims >= 1 && count > 0) {
     Method m = choose_method(*r, count);
-    err = start_isend(*r, m, p.device_ptr, count, dest, tag, comm, request);
+    err = start_isend(*r, m, p, count, dest, tag, comm, request);
   } else {
     // earlier managed sends reach the library first (non-overtaking)
     err = progress_sends();
@@ -339,7 +339,7 @@ int MPI_Irecv(void *buf, int count, MPI_Datatype datatype, int source, int tag,
   int err;
   if (r && r->packable && r->desc.ndims >= 1 && count > 0) {
     Method m = choose_method(*r, count);
-    err = start_irecv(*r, m, p.device_ptr, count, source, tag, comm, request);
+    err = start_irecv(*r, m, p, count, source, tag, comm, request);
   } else {
     err = libmpi.Irecv(buf, count, datatype, source, tag, comm, request);
   }

@@ -44,6 +44,10 @@ int sync(cudaStream_t s) {
                           : cuda_error(e, "stream synchronize");
 }
 
+// launch_geometry's both_device for the user's buffer and a host slab (with a
+// device slab it is whether the buffer is device memory)
+int with_host(const PtrInfo &buf) { return buf.is_host ? kBothHost : 0; }
+
 void *host_dev_ptr(void *h) {
   void *d = nullptr;
   if (cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
@@ -55,8 +59,8 @@ void *host_dev_ptr(void *h) {
 
 } // namespace
 
-int send_strided(TypeRecord &r, Method m, const void *buf, int count, int dest,
-                 int tag, MPI_Comm comm) {
+int send_strided(TypeRecord &r, Method m, const PtrInfo &buf, int count,
+                 int dest, int tag, MPI_Comm comm) {
   const int64_t bytes = int64_t(count) * r.desc.size;
   cudaStream_t s = pack_stream();
   tempi_config cfg = choose_config(r, count, false, m == Method::ONESHOT,
@@ -68,7 +72,8 @@ int send_strided(TypeRecord &r, Method m, const void *buf, int count, int dest,
     void *h = slab_alloc(Space::HOST_MAPPED, bytes);
     if (!h)
       return MPI_ERR_NO_MEM;
-    err = tempi_pack(&r.desc, buf, count, host_dev_ptr(h), &cfg, s);
+    err = pack_known(&r.desc, buf.device_ptr, count, host_dev_ptr(h), &cfg, s,
+                     with_host(buf));
     if (!err)
       err = sync(s);
     int merr = err ? to_mpi(err)
@@ -85,7 +90,7 @@ int send_strided(TypeRecord &r, Method m, const void *buf, int count, int dest,
       slab_free(Space::HOST_MAPPED, h);
       return MPI_ERR_NO_MEM;
     }
-    err = tempi_pack(&r.desc, buf, count, d, &cfg, s);
+    err = pack_known(&r.desc, buf.device_ptr, count, d, &cfg, s, buf.is_device);
     if (!err) {
       cudaError_t e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s);
       err = e == cudaSuccess ? sync(s) : cuda_error(e, "staged copy");
@@ -101,7 +106,7 @@ int send_strided(TypeRecord &r, Method m, const void *buf, int count, int dest,
     void *d = slab_alloc(Space::DEVICE, bytes);
     if (!d)
       return MPI_ERR_NO_MEM;
-    err = tempi_pack(&r.desc, buf, count, d, &cfg, s);
+    err = pack_known(&r.desc, buf.device_ptr, count, d, &cfg, s, buf.is_device);
     if (!err)
       err = sync(s);
     int merr = err ? to_mpi(err)
@@ -112,8 +117,8 @@ int send_strided(TypeRecord &r, Method m, const void *buf, int count, int dest,
   }
 }
 
-int recv_strided(TypeRecord &r, Method m, void *buf, int count, int source,
-                 int tag, MPI_Comm comm, MPI_Status *status) {
+int recv_strided(TypeRecord &r, Method m, const PtrInfo &buf, int count,
+                 int source, int tag, MPI_Comm comm, MPI_Status *status) {
   const int64_t bytes = int64_t(count) * r.desc.size;
   cudaStream_t s = pack_stream();
   tempi_config cfg = choose_config(r, count, false, m == Method::ONESHOT,
@@ -128,7 +133,8 @@ int recv_strided(TypeRecord &r, Method m, void *buf, int count, int source,
     int merr =
         libmpi.Recv(h, int(bytes), MPI_PACKED, source, tag, comm, status);
     if (merr == MPI_SUCCESS) {
-      err = tempi_unpack(&r.desc, host_dev_ptr(h), count, buf, &cfg, s);
+      err = unpack_known(&r.desc, host_dev_ptr(h), count, buf.device_ptr, &cfg, s,
+                         with_host(buf));
       if (!err)
         err = sync(s);
       merr = to_mpi(err);
@@ -149,8 +155,10 @@ int recv_strided(TypeRecord &r, Method m, void *buf, int count, int source,
         libmpi.Recv(h, int(bytes), MPI_PACKED, source, tag, comm, status);
     if (merr == MPI_SUCCESS) {
       cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
-      err = e == cudaSuccess ? tempi_unpack(&r.desc, d, count, buf, &cfg, s)
-                             : cuda_error(e, "staged copy");
+      err = e == cudaSuccess
+                ? unpack_known(&r.desc, d, count, buf.device_ptr, &cfg, s,
+                               buf.is_device)
+                : cuda_error(e, "staged copy");
       if (!err)
         err = sync(s);
       merr = to_mpi(err);
@@ -167,7 +175,8 @@ int recv_strided(TypeRecord &r, Method m, void *buf, int count, int source,
     int merr =
         libmpi.Recv(d, int(bytes), MPI_PACKED, source, tag, comm, status);
     if (merr == MPI_SUCCESS) {
-      err = tempi_unpack(&r.desc, d, count, buf, &cfg, s);
+      err = unpack_known(&r.desc, d, count, buf.device_ptr, &cfg, s,
+                         buf.is_device);
       if (!err)
         err = sync(s);
       merr = to_mpi(err);
@@ -234,7 +243,7 @@ class IsendOp : public AsyncOp {
 
 public:
   int err = MPI_SUCCESS;
-  IsendOp(TypeRecord &r, Method m, const void *buf, int count, int dest,
+  IsendOp(TypeRecord &r, Method m, const PtrInfo &buf, int count, int dest,
           int tag, MPI_Comm comm)
       : m_(m) {
     const int64_t bytes = int64_t(count) * r.desc.size;
@@ -251,12 +260,14 @@ public:
       host_ = slab_alloc(Space::HOST_MAPPED, bytes);
       packed = host_;
       if (host_)
-        terr = tempi_pack(&r.desc, buf, count, host_dev_ptr(host_), &cfg, s);
+        terr = pack_known(&r.desc, buf.device_ptr, count, host_dev_ptr(host_),
+                          &cfg, s, with_host(buf));
     } else {
       dev_ = slab_alloc(Space::DEVICE, bytes);
       packed = dev_;
       if (dev_)
-        terr = tempi_pack(&r.desc, buf, count, dev_, &cfg, s);
+        terr = pack_known(&r.desc, buf.device_ptr, count, dev_, &cfg, s,
+                          buf.is_device);
       if (m == Method::STAGED && dev_ && !terr) {
         host_ = slab_alloc(Space::HOST_MAPPED, bytes);
         packed = host_;
@@ -316,7 +327,7 @@ public:
 class IrecvOp : public AsyncOp {
   TypeRecord &r_;
   Method m_;
-  void *buf_;
+  PtrInfo buf_;
   int count_;
   void *dev_ = nullptr, *host_ = nullptr;
   MPI_Request req_ = MPI_REQUEST_NULL;
@@ -326,7 +337,7 @@ class IrecvOp : public AsyncOp {
 
 public:
   int err = MPI_SUCCESS;
-  IrecvOp(TypeRecord &r, Method m, void *buf, int count, int source, int tag,
+  IrecvOp(TypeRecord &r, Method m, const PtrInfo &buf, int count, int source, int tag,
           MPI_Comm comm)
       : r_(r), m_(m), buf_(buf), count_(count) {
     const int64_t bytes = int64_t(count) * r.desc.size;
@@ -368,7 +379,8 @@ public:
                                    true);
     int terr = TEMPI_OK;
     if (m_ == Method::ONESHOT) {
-      terr = tempi_unpack(&r_.desc, host_dev_ptr(host_), count_, buf_, &cfg, s);
+      terr = unpack_known(&r_.desc, host_dev_ptr(host_), count_,
+                          buf_.device_ptr, &cfg, s, with_host(buf_));
     } else {
       if (m_ == Method::STAGED) {
         cudaError_t e =
@@ -377,7 +389,8 @@ public:
           terr = cuda_error(e, "staged copy");
       }
       if (!terr)
-        terr = tempi_unpack(&r_.desc, dev_, count_, buf_, &cfg, s);
+        terr = unpack_known(&r_.desc, dev_, count_, buf_.device_ptr, &cfg, s,
+                            buf_.is_device);
     }
     if (!terr && cudaEventRecord(ev_, s) != cudaSuccess)
       terr = cuda_error(cudaGetLastError(), "event record");
@@ -441,7 +454,7 @@ MPI_Request make_request() {
 
 } // namespace
 
-int start_isend(TypeRecord &r, Method m, const void *buf, int count, int dest,
+int start_isend(TypeRecord &r, Method m, const PtrInfo &buf, int count, int dest,
                 int tag, MPI_Comm comm, MPI_Request *request) {
   auto op = std::make_unique<IsendOp>(r, m, buf, count, dest, tag, comm);
   if (op->err)
@@ -454,7 +467,7 @@ int start_isend(TypeRecord &r, Method m, const void *buf, int count, int dest,
   return MPI_SUCCESS;
 }
 
-int start_irecv(TypeRecord &r, Method m, void *buf, int count, int source,
+int start_irecv(TypeRecord &r, Method m, const PtrInfo &buf, int count, int source,
                 int tag, MPI_Comm comm, MPI_Request *request) {
   auto op = std::make_unique<IrecvOp>(r, m, buf, count, source, tag, comm);
   if (op->err)
