@@ -387,7 +387,7 @@ __device__ __forceinline__ void store_end(char *w, const uint4 &v, uint32_t a,
 }
 
 template <int U, int ND, bool UNPACK>
-__global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 6)
+__global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 8)
     k_realign(char *__restrict__ strided, char *__restrict__ packed,
               const __grid_constant__ Geometry g,
               const __grid_constant__ Realign r) {
@@ -1122,21 +1122,24 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t sbase,
 
 // Whether the realign kernel takes a launch whose kernel the library chooses
 // (device memory on both sides).  Measured on B200 by synchronised calls over
-// 590 random layouts whose rows are not 16-byte words, against the kernel the
-// cost model or the fixed rules pick (its time / the realign kernel's, mean):
+// 650 random layouts whose rows are not 16-byte words, three buffer sets in
+// turn, against the kernel the cost model picks (its time / the realign
+// kernel's, mean):
 //  * rows of 8 KiB and more in 32 MiB and more (contiguous runs among them):
-//    1.06 for 4- and 8-byte words, 1.5 for narrower ones (a 60 MB run at an
+//    1.03 for 4- and 8-byte words, 1.5 for narrower ones (a 60 MB run at an
 //    odd offset 54 -> 30 us);
-//  * odd rows (1- and 2-byte words) of 4 KiB and more, too few to give every
-//    SM 16 warps a row each, from 2 MB: 1.07 to 1.3 (4-byte words of 8 KiB
-//    rows from 16 MB: 1.2, where the pick is a kernel by rows);
-//  * short odd rows: packs below 128 B from 2 MB 1.08 to 1.5, unpacks of 64
-//    to 255 B from 4 MB 1.02 to 1.26;
+//  * odd rows (1- and 2-byte words) of 4 KiB and more from 1 MB: 1.03 to 1.05
+//    up to 2 MB, 1.07 to 1.13 to 8 MB, 1.3 to 1.5 beyond (rows of 4 to 8 KiB
+//    only while they are too few to give every SM 16 warps a row each; 4-byte
+//    words of 8 KiB rows likewise from 16 MB, 1.2);
+//  * short odd rows: packs of up to 127 B from 2 MB 1.07 to 1.4, of up to 255 B
+//    from 4 MB 1.06, unpacks of 64 to 255 B from 2 MB 1.02 to 1.4;
 //  * unpacks of 64-B to 2-KiB rows that cut sectors, in more than the L2 keeps
 //    (cuts_sectors below): 1.02 to 1.4.
-// Between these, odd rows of 256 B to 4 KiB run 3 to 9 % faster with a group
+// Between these, odd rows of 256 B to 4 KiB run 0 to 8 % faster with a group
 // of lanes per row (the shift kernel), and 4- and 8-byte words of rows the
-// L2 holds with the word kernels, whose few instructions cost less latency.
+// L2 holds 3 to 8 % faster with the word and row kernels, whose few
+// instructions cost less latency.
 static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack,
                          bool cut, int sms) {
   if (cut)
@@ -1151,9 +1154,11 @@ static bool realign_wins(const Geometry &g, uint64_t bytes, bool unpack,
   if (g.width > 2)
     return false;
   if (g.block >= 4096)
-    return g.rows < uint32_t(16 * sms) && bytes >= 2 * MB;
-  return unpack ? g.block >= 64 && g.block < 256 && bytes >= 4 * MB
-                : g.block < 128 && bytes >= 2 * MB;
+    return bytes >= 1 * MB &&
+           (g.block >= 8192 || g.rows < uint32_t(16 * sms));
+  if (unpack)
+    return g.block >= 64 && g.block < 256 && bytes >= 2 * MB;
+  return g.block < 128 ? bytes >= 2 * MB : g.block < 256 && bytes >= 4 * MB;
 }
 
 // Whether an unpack's rows leave partial sectors in lines that the L2 will not
@@ -1196,12 +1201,12 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
     r.div = make_fastdiv(uint32_t(g.block));
     r.words = uint32_t((uint64_t(a0) + r.bytes + 15) / 16);
   }
-  // one word a thread for small objects and short rows (less code to fetch,
-  // more warps), four for long streams (10 % faster from 32 MB on) and for
-  // longer rows with cut ends (up to 10 % from 256 B on)
+  // one word a thread for small objects and short rows (less code to fetch, 64
+  // warps an SM), four for long streams (5 % faster from 32 MB on) and for
+  // longer rows with cut ends (4 to 6 % from 700 B on)
   const int asked = cfg && cfg->kernel == 5 ? cfg->unroll : 0;
   const uint32_t words = asked == 1 || asked == 4 ? uint32_t(asked)
-                         : r.bytes >= 8000000u && g.block >= (cut ? 256 : 4096)
+                         : r.bytes >= 8000000u && g.block >= (cut ? 512 : 4096)
                              ? 4u
                              : 1u;
   const uint32_t per = uint32_t(kRealignThreads) * words;

@@ -72,17 +72,18 @@ def test_dimensions(cuda, mpi_init, nd):
 
 
 @pytest.mark.parametrize("start,block,counts,strides,kernels", [
-    (3, 2_000_001, [], [], ("realign", "realign")),        # a long odd run
-    (3, 1_999_999, [], [], ("words", "words")),            # just too small for it
+    (3, 1_000_001, [], [], ("realign", "realign")),        # a long odd run
+    (3, 999_999, [], [], ("words", "words")),              # just too small for it
     (4, 33_554_436, [], [], ("realign", "realign")),       # 4-byte words from 32 MiB
     (4, 33_554_428, [], [], ("words", None)),
-    (1, 127, [15_800], [130], ("realign", None)),          # short odd rows, packed
-    (1, 128, [15_800], [131], (None, None)),
-    (1, 130, [31_000], [133], (None, "realign")),          # and unpacked
-    (1, 63, [64_000], [66], ("realign", None)),
+    (1, 127, [15_800], [130], ("realign", "realign")),     # short odd rows, 2 MB
+    (1, 63, [32_000], [66], ("realign", None)),
+    (1, 128, [15_800], [131], (None, "realign")),
+    (1, 129, [31_100], [133], ("realign", "realign")),     # ... packs of up to 255 B, 4 MB
     (1, 256, [16_000], [259], (None, None)),
     (1, 4097, [2300], [4101], ("realign", "realign")),     # too few rows for a warp each
     (1, 4097, [2400], [4101], (None, None)),
+    (1, 8193, [2400], [8201], ("realign", "realign")),
     (4, 260, [93_000], [264], (None, "realign")),          # rows that cut sectors, 60.3 MB
     (4, 260, [92_000], [264], (None, None)),               # ... 59.6 MB
     (2, 262, [74_000], [266], (None, "realign")),          # ... 48.2 MB of 2-byte words
