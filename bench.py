@@ -352,7 +352,10 @@ def learned_configs(lib, d, n):
                                          ctypes.byref(uc), ctypes.byref(mi), None, None))
     out = []
     for k in (pc.value, uc.value):
-        out.append(_lib.Config(*_lib.CANDIDATE_CONFIGS[k]) if k >= 0 else None)
+        cfg = _lib.Config(*_lib.CANDIDATE_CONFIGS[k]) if k >= 0 else None
+        if cfg:
+            cfg.reserved = _lib.OWN_CHOICE
+        out.append(cfg)
     return out
 
 

@@ -94,6 +94,10 @@ CANDIDATE_CONFIGS = (
     (3, 0, 256, 4, 0, 0), (3, 0, 256, 8, 0, 0), (3, 0, 256, 16, 0, 0), (3, 0, 256, 32, 0, 0),
     (4, 0, 256, 0, 3, 0), (4, 0, 256, 0, 8, 0),
 )
+# The dispatcher's mark on them (kOwnChoice in csrc/tempi/internal.hpp), in
+# ``reserved``: a rule of the library may still put another kernel in their
+# place, as it may under MPI_Pack; without it the asked-for kernel runs.
+OWN_CHOICE = 0x7E91
 
 
 class Region(ctypes.Structure):
