@@ -1550,7 +1550,8 @@ extern "C" int tempi_batch_config(const tempi_batch *b, int32_t *threads,
 // refreshed if the application resets the device (cudaDeviceReset).
 //
 // A table of up to kParamRegions entries is passed BY VALUE as the batch
-// kernel's own parameter (k_batch_param): one launch, the array untouched.
+// kernel's own parameter (k_batch_param_small, or k_batch_param where a region
+// has more than two strided dimensions): one launch, the array untouched.
 // A larger table reaches the array without a host-to-device copy: the host
 // builds it in pieces of up to kFillPiece entries and passes each piece BY
 // VALUE as the parameter of a small kernel (k_static_fill) that writes it
