@@ -1231,6 +1231,9 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
 // where they are, for the grids below (smaller ones fit them anyway).
 constexpr uint64_t kLinkMinBytes = uint64_t(512) << 10;
 
+// Packed bytes from which the dispatcher's staged picks run as such.
+constexpr uint64_t kStagedMinBytes = 16000000;
+
 // Rows that the shift and row kernels take once each (launch_geometry).
 constexpr int64_t kOnceMinRow = 64, kOnceMaxRow = 4096;
 constexpr uint64_t kOnceRowsBytes = 32000000;
@@ -1254,6 +1257,24 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
     if (both_device == 1)
       return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
                             cfg, stream);
+  }
+  // A staged kernel's bytes go through shared memory before the first store:
+  // about 1.2 us more latency, which long streams make up for and a call that
+  // is waited for does not below 16 MB (8 MB for rows below 64 B).  Where the
+  // dispatcher, whose model knows launches back to back, picks it there, the
+  // word kernel runs.  Synchronised, over 54 unpacks of 4- to 16-byte words:
+  // 1.08 to 1.15 up to 4 MB (13.0 -> 11.6 us), 1.03 to 1.12 up to 8 MB, 1.04 to
+  // 1.10 up to 16 MB (rows below 64 B 1.02, from 0.95 to 1.09), 0.97 to 1.02
+  // beyond; over 14 packs of 16-byte words 1.10 up to 16 MB, 1.01 beyond (of
+  // narrower ones the staged kernels take none).
+  if (kernel == 4 && own && g.width >= (unpack ? 4u : 16u) &&
+      uint64_t(g.rows) * uint64_t(g.block) <
+          (g.block < 64 ? kStagedMinBytes / 2 : kStagedMinBytes) &&
+      (both_device >= 0
+           ? both_device == 1
+           : classify(strided).is_device && classify(packed).is_device)) {
+    kernel = 1;
+    cfg = nullptr; // its launch shape is the staged kernel's
   }
   // the staged kernels (4), where their bulk copies are allowed: unpack
   // needs a 16-B aligned packed base and a packed size that is a multiple of
