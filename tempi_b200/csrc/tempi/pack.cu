@@ -1266,8 +1266,10 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // 1.08 to 1.15 up to 4 MB (13.0 -> 11.6 us), 1.03 to 1.12 up to 8 MB, 1.04 to
   // 1.10 up to 16 MB (rows below 64 B 1.02, from 0.95 to 1.09), 0.97 to 1.02
   // beyond; over 14 packs of 16-byte words 1.10 up to 16 MB, 1.01 beyond (of
-  // narrower ones the staged kernels take none).
-  if (kernel == 4 && own && g.width >= (unpack ? 4u : 16u) &&
+  // narrower ones the staged kernels take none).  Not 4-byte words of rows below
+  // 64 B: 262,144 rows of 16 B 6.4 us in-kernel staged, 7.1 by words.
+  if (kernel == 4 && own &&
+      g.width >= (!unpack ? 16u : g.block < 64 ? 8u : 4u) &&
       uint64_t(g.rows) * uint64_t(g.block) <
           (g.block < 64 ? kStagedMinBytes / 2 : kStagedMinBytes) &&
       (both_device >= 0

@@ -1,7 +1,7 @@
 """Where the dispatcher picks the staged kernels, the word kernel runs below
-16 MB (8 MB for rows below 64 B) of 4-byte and wider words in device memory:
-both sides of each line, the widths it holds for and one it does not, and the
-staged kernel where a caller asks for it by number."""
+16 MB of 4-byte and wider words in device memory (8 MB of 8-byte and wider ones
+for rows below 64 B): both sides of each line, the widths it holds for and ones
+it does not, and the staged kernel where a caller asks for it by number."""
 import ctypes
 
 import pytest
@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("mine", [True, False])
 @pytest.mark.parametrize("block,rows,gap,words", [
-    (16, 499_999, 32, True), (16, 500_000, 32, False), (60, 66_668, 4, True),
+    (16, 499_999, 32, True), (16, 500_000, 32, False), (60, 66_668, 4, False),
+    (56, 71_428, 8, True),
     (64, 249_999, 64, True), (64, 250_000, 64, False), (4096, 3, 16, True),
     (8_000_008, 1, 0, True), (15_999_984, 1, 0, True), (16_000_000, 1, 0, False),
     (72, 27_776, 56, True), (254, 8_000, 2, False),
