@@ -37,6 +37,7 @@
 //  * grids are a multiple of the SM count and grid-stride over the work.
 
 #include "internal.hpp"
+#include "realign.hpp"
 #include "runtime.hpp"
 
 #include <algorithm>
@@ -302,7 +303,6 @@ __global__ void __launch_bounds__(256)
 // when the rows are sector-aligned).  Long streams are bound by DRAM: a 60 MB run at an odd
 // offset packs in 20 us beyond the call's fixed cost, 0.92 of the copy peak
 // (the word kernel, at a byte a thread: 44 us).
-constexpr int64_t kRealignMinRow = 16; // a packed word touches at most two rows
 constexpr int kRealignThreads = 256;
 
 struct Realign {
@@ -324,8 +324,8 @@ __device__ __forceinline__ uint32_t load_pair(const char *base, int off, int n,
   const uint32_t m = uint32_t(reinterpret_cast<uintptr_t>(p) & 15);
   const uint4 *q = reinterpret_cast<const uint4 *>(p - m);
   const int lo = off - int(m); // of the first word, relative to base
-  *a = lo > -16 && lo < n ? __ldg(q) : make_uint4(0, 0, 0, 0);
-  *b = m && lo > -32 && lo + 16 < n ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
+  *a = word_holds(lo, n) ? __ldg(q) : make_uint4(0, 0, 0, 0);
+  *b = m && next_word_holds(lo, n) ? __ldg(q + 1) : make_uint4(0, 0, 0, 0);
   return m;
 }
 
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 8)
         continue;
       }
       if (!UNPACK) {
-        const int p = int(16 * t - a0);
+        const int p = packed_word(t, a0);
         const uint32_t row = fastdiv(p < 0 ? 0u : uint32_t(p), r.div);
         at[u] = p - int(row) * n;
         m[u] = load_pair(strided + row_offset<ND>(row, g), at[u], n, &a[u], &b[u]);
@@ -417,13 +417,12 @@ __global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 8)
         const uint32_t row = fastdiv(t, r.div), j = t - row * r.div.d;
         char *d = strided + row_offset<ND>(row, g);
         const uint32_t lo = uint32_t(reinterpret_cast<uintptr_t>(d) & 15);
-        at[u] = int(16 * j) - int(lo);
-        if (at[u] >= n) {
+        if (!slot_in_row(j, lo, n, &at[u])) {
           at[u] = 0x7fffffff;
           continue;
         }
         to[u] = d + at[u];
-        if (r.edges && (at[u] <= 0 || at[u] + 16 >= n))
+        if (r.edges && (at[u] <= 0 || at[u] >= n - 16))
           fetch_line(at[u] < 0 ? d : to[u]);
         m[u] = load_pair(packed, int(row) * n + at[u], total, &a[u], &b[u]);
       }
@@ -434,9 +433,9 @@ __global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 8)
         continue;
       uint4 v = cut16(a[u], b[u], m[u]);
       if (!UNPACK) {
-        const int p = int(16 * (t0 + u * blockDim.x) - a0);
-        const int k = n - at[u]; // bytes this row still has
-        if (k < 16 && p + k < total) {
+        const int p = packed_word(t0 + u * blockDim.x, a0);
+        if (!ends_within(at[u], n) && n - at[u] < total - p) {
+          const int k = n - at[u]; // bytes this row still has
           const uint32_t row = fastdiv(p < 0 ? 0u : uint32_t(p), r.div) + 1;
           uint4 c, d;
           const uint32_t mm =
@@ -444,17 +443,17 @@ __global__ void __launch_bounds__(kRealignThreads, U == 4 ? 4 : 8)
           v = join(v, cut16(c, d, mm), k);
         }
         char *w = packed + p;
-        if (p >= 0 && p + 16 <= total)
+        if (p >= 0 && ends_within(p, total))
           *reinterpret_cast<uint4 *>(w) = v;
         else
           store_part(w, v, p < 0 ? uint32_t(-p) : 0u,
-                     p + 16 <= total ? 16u : uint32_t(total - p)); // once a pack
+                     ends_within(p, total) ? 16u : uint32_t(total - p)); // once a pack
       } else {
-        if (at[u] >= 0 && at[u] + 16 <= n)
+        if (at[u] >= 0 && ends_within(at[u], n))
           *reinterpret_cast<uint4 *>(to[u]) = v;
         else
           store_end(to[u], v, at[u] < 0 ? uint32_t(-at[u]) : 0u,
-                    at[u] + 16 <= n ? 16u : uint32_t(n - at[u]));
+                    ends_within(at[u], n) ? 16u : uint32_t(n - at[u]));
       }
     }
   }
@@ -1193,13 +1192,13 @@ static int launch_realign(const Geometry &g, char *strided, char *packed,
   r.edges = cut;
   if (unpack) {
     // destination words a row can touch, whatever its alignment
-    const uint32_t slots = uint32_t((g.block + 30) / 16);
+    const uint32_t slots = row_slots(uint32_t(g.block));
     r.div = make_fastdiv(slots);
     r.words = g.rows * slots;
   } else {
     const uint32_t a0 = uint32_t(reinterpret_cast<uintptr_t>(packed) & 15);
     r.div = make_fastdiv(uint32_t(g.block));
-    r.words = uint32_t((uint64_t(a0) + r.bytes + 15) / 16);
+    r.words = packed_words(r.bytes, a0);
   }
   // one word a thread for small objects and short rows (less code to fetch, 64
   // warps an SM), four for long streams (5 % faster from 32 MB on) and for
