@@ -1396,6 +1396,10 @@ extern "C" int tempi_batch_tune(tempi_batch *b, void *stream, int32_t reps) {
     return TEMPI_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   reps = std::max(1, std::min(50, int(reps)));
+  // Launches of this batch may be in flight on any stream; they read the table
+  // that every plan below rewrites.
+  if (cudaDeviceSynchronize() != cudaSuccess)
+    return cuda_error(cudaGetLastError(), "tuning: launches before it");
   drop_graph(bi);
   int dev = 0, l2 = 0;
   cudaGetDevice(&dev);
