@@ -316,7 +316,9 @@ const char *tempi_last_kernel(void);
    slabs held from CUDA), "slab_live_bytes" (handed out), "slab_cached_bytes"
    (kept for reuse, at most TEMPI_SLAB_CACHE_MB per memory space),
    "host_link_copies", "send_contig_staged", "recv_contig_staged",
-   "neighbor_fused", "neighbor_isir", "neighbor_lib", "alltoallv_staged",
+   "neighbor_fused", "neighbor_isir", "neighbor_lib", "neighbor_uploads" (region
+   tables that a fused MPI_Neighbor_alltoallw copied to the device),
+   "alltoallv_staged",
    "alltoallv_remote_first", "alltoallv_isir_staged",
    "alltoallv_isir_remote_staged", "alltoallv_lib", and "staged_timeouts"
    (staged launches whose bounded waits gave up, as far as the host has seen:

@@ -1211,13 +1211,17 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
 // One copy batch on `s`.  Up to kParamRegions pairs of at most two strided
 // dimensions (a halo's 26) travel in the kernel's parameters: nothing is
 // uploaded, whatever regions the previous call had.  Larger tables go to a
-// grow-only device buffer: no allocation once it is large enough.  The caller
-// synchronises `s` before the next call (the table is rewritten by every
-// call).
+// grow-only device buffer: no allocation once it is large enough, and no copy
+// while it holds the same entries byte for byte (a loop that exchanges the same
+// regions every step uploads them once: 33 edges 15.7 us a call, 18.4 with the
+// copy; 200 edges 32.7 and 35.5; 26 edges of three strided dimensions 17.3 and
+// 20.0).  Every call is on `s`, TEMPI's one stream, so a new table is copied
+// behind the launches that read the old one.
 int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
   static std::mutex mu;
   static void *table = nullptr;
   static size_t capacity = 0; // bytes
+  static std::vector<char> on_device; // the entries in the table
   static std::vector<CopyPair> pairs;
   std::lock_guard<std::mutex> l(mu);
   std::unique_lock<std::mutex> tuning(g_tune_mu);
@@ -1269,14 +1273,21 @@ int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
     cudaFree(table);
     table = nullptr;
     capacity = 0;
+    on_device.clear();
     cudaError_t e = cudaMalloc(&table, bytes);
     if (e != cudaSuccess)
       return cuda_error(e, "copy table allocation");
     capacity = bytes;
   }
-  cudaError_t e = cudaMemcpyAsync(table, from, bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess)
-    return cuda_error(e, "copy table upload");
+  const char *b = static_cast<const char *>(from);
+  if (on_device.size() != bytes || std::memcmp(on_device.data(), b, bytes) != 0) {
+    on_device.clear();
+    cudaError_t e = cudaMemcpyAsync(table, from, bytes, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess)
+      return cuda_error(e, "copy table upload");
+    on_device.assign(b, b + bytes);
+    counters().neighbor_uploads++;
+  }
   return launch_table<CopyPair>(table, count, small, uint32_t(chunks), 0, shape, s,
                                 false);
 }
