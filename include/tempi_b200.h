@@ -318,6 +318,7 @@ const char *tempi_last_kernel(void);
    "host_link_copies", "send_contig_staged", "recv_contig_staged",
    "neighbor_fused", "neighbor_isir", "neighbor_lib", "neighbor_uploads" (region
    tables that a fused MPI_Neighbor_alltoallw copied to the device),
+   "neighbor_tables" (allocations of the memory they are copied to),
    "alltoallv_staged",
    "alltoallv_remote_first", "alltoallv_isir_staged",
    "alltoallv_isir_remote_staged", "alltoallv_lib", and "staged_timeouts"

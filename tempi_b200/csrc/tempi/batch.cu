@@ -1220,6 +1220,9 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
 int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
   static std::mutex mu;
   static void *table = nullptr;
+  // room for 64 full entries or 164 compact ones, so that exchanges of a few
+  // more edges each do not free and allocate every time
+  constexpr size_t kLeastTable = 64 * sizeof(CopyPair);
   static size_t capacity = 0; // bytes
   static std::vector<char> on_device; // the entries in the table
   static std::vector<CopyPair> pairs;
@@ -1274,10 +1277,12 @@ int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
     table = nullptr;
     capacity = 0;
     on_device.clear();
-    cudaError_t e = cudaMalloc(&table, bytes);
+    const size_t want = std::max(bytes, kLeastTable);
+    cudaError_t e = cudaMalloc(&table, want);
     if (e != cudaSuccess)
       return cuda_error(e, "copy table allocation");
-    capacity = bytes;
+    capacity = want;
+    counters().neighbor_tables++;
   }
   const char *b = static_cast<const char *>(from);
   if (on_device.size() != bytes || std::memcmp(on_device.data(), b, bytes) != 0) {

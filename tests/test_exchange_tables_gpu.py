@@ -81,3 +81,16 @@ def test_unchanged_tables_are_copied_once(cuda, mpi_init, edges, dims):
     assert _lib.counter("neighbor_uploads") == n + 4
     mpi.Comm_free(x.comm)
     mpi.Comm_free(other.comm)
+
+
+def test_growing_exchanges_share_an_allocation(cuda, mpi_init):
+    """From 33 edges to 64, one more at a time: at most one allocation (none if
+    an earlier exchange of the process had as many)."""
+    t, extent = hvectors(8, [(3, 8)])
+    n = _lib.counter("neighbor_tables")
+    assert n >= 0
+    for edges in range(33, 65):
+        x = Exchange(t, extent, edges)
+        x.run()
+        mpi.Comm_free(x.comm)
+    assert _lib.counter("neighbor_tables") <= n + 1
