@@ -319,6 +319,7 @@ const char *tempi_last_kernel(void);
    "neighbor_fused", "neighbor_isir", "neighbor_lib", "neighbor_uploads" (region
    tables that a fused MPI_Neighbor_alltoallw copied to the device),
    "neighbor_tables" (allocations of the memory they are copied to),
+   "neighbor_unit" (such calls served from what the types' commit settled),
    "alltoallv_staged",
    "alltoallv_remote_first", "alltoallv_isir_staged",
    "alltoallv_isir_remote_staged", "alltoallv_lib", and "staged_timeouts"

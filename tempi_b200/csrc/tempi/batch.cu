@@ -849,11 +849,11 @@ void load_tuned_locked() {
 
 // signature of a batch: what kind of launch it is, and the multiset of its
 // records' (class, log2 words)
-template <typename Rec> uint64_t signature(const std::vector<Rec> &recs, int unpack) {
+template <typename Rec> uint64_t signature(const Rec *recs, size_t n, int unpack) {
   std::vector<uint32_t> keys;
-  keys.reserve(recs.size());
-  for (const Rec &r : recs) {
-    const Geometry &g = geometry_of(r);
+  keys.reserve(n);
+  for (size_t i = 0; i < n; ++i) {
+    const Geometry &g = geometry_of(recs[i]);
     keys.push_back(uint32_t(region_class(g)) << 8 | uint32_t(ilog2(g.total_words)));
   }
   std::sort(keys.begin(), keys.end());
@@ -870,13 +870,31 @@ template <typename Rec> uint64_t signature(const std::vector<Rec> &recs, int unp
   return h;
 }
 
-// the passes of every record from `t` (or the defaults) and the chunk count
+// passes of a region class from `t` (or the default)
+uint32_t passes_of(int cls, const Tuned *t) {
+  return t && t->passes[cls] ? t->passes[cls] : default_passes(cls);
+}
+
+// The choices tuned for this signature, if any; no signature is formed while
+// nothing is tuned at all.
+template <typename Rec>
+bool find_tuned(const Rec *recs, size_t n, int unpack, Tuned *out) {
+  std::lock_guard<std::mutex> l(g_tune_mu);
+  load_tuned_locked();
+  if (g_tuned.empty())
+    return false;
+  auto it = g_tuned.find(signature(recs, n, unpack));
+  if (it == g_tuned.end())
+    return false;
+  *out = it->second;
+  return true;
+}
+
+// the passes of every record and the chunk count
 template <typename Rec>
 uint64_t apply_passes(std::vector<Rec> &recs, const Tuned *t) {
-  for (Rec &r : recs) {
-    const int c = region_class(geometry_of(r));
-    r.passes = t && t->passes[c] ? t->passes[c] : default_passes(c);
-  }
+  for (Rec &r : recs)
+    r.passes = passes_of(region_class(geometry_of(r)), t);
   return assign_chunks(recs);
 }
 
@@ -909,7 +927,7 @@ using namespace tempi;
 // records' passes and chunks, returns the chunk total
 template <typename Rec>
 static uint64_t plan_batch(BatchImpl &bi, std::vector<Rec> &recs) {
-  bi.sig = signature(recs, bi.unpack);
+  bi.sig = signature(recs.data(), recs.size(), bi.unpack);
   {
     std::lock_guard<std::mutex> l(g_tune_mu);
     load_tuned_locked();
@@ -1045,6 +1063,11 @@ __global__ void __launch_bounds__(256, kSmallThreadsPerSm / 256)
   small_chunks<false>(in_memory(piece.r), npairs, total_chunks, 1, s_begin);
 }
 
+// whether a tuned shape is one that the kernels with a parameter table have
+static bool param_shape(const Shape &s) {
+  return s.threads == 0 || s.threads == 256;
+}
+
 // k_batch_param(_small) over the `n` <= kParamRegions entries of `table`
 // (host memory), `per_sm` CTAs per SM (0: as many as fit)
 template <typename Rec>
@@ -1175,14 +1198,15 @@ namespace tempi {
 // most two strided dimensions (a halo's 26 regions): entries straight from the
 // geometries settled when the types were committed, no division of lengths and
 // no descriptors copied (a 256^3 exchange: 4.1 us less host time a call, with
-// the types looked up under one lock).  False when some edge is not of this
-// kind.
+// the types looked up under one lock).  An exchange whose own signature was
+// tuned takes its passes and shape; what else was tuned changes nothing.
+// False when some edge is not of this kind, or the tuned shape needs another
+// kernel.
 static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
                                int *err) {
   if (n > kParamRegions)
     return false;
-  SmallPair entries[kParamRegions];
-  uint64_t chunks = 0;
+  CopyPair pairs[kParamRegions];
   for (int i = 0; i < n; ++i) {
     const CopyEdge &e = edges[i];
     const TypeRecord &a = *e.src_type, &b = *e.dst_type;
@@ -1195,16 +1219,28 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
                                    reinterpret_cast<uintptr_t>(dst)) |
                           a.unit[4].width | b.unit[4].width;
     const int k = __builtin_ctz(bits); // the width both sides prove: 2^k <= 16
-    CopyPair p{src, dst, a.unit[k], b.unit[k], uint32_t(chunks), 0};
-    p.passes = default_passes(region_class(p.gs));
+    pairs[i] = {src, dst, a.unit[k], b.unit[k], 0, 0};
+  }
+  Tuned tuned;
+  const bool has_tuned = find_tuned(pairs, size_t(n), 0, &tuned);
+  if (has_tuned && !param_shape(tuned.shape))
+    return false;
+  SmallPair entries[kParamRegions];
+  uint64_t chunks = 0;
+  for (int i = 0; i < n; ++i) {
+    CopyPair &p = pairs[i];
+    p.chunk_begin = uint32_t(chunks);
+    p.passes = passes_of(region_class(p.gs), has_tuned ? &tuned : nullptr);
     entries[i] = make_small(p);
     chunks += chunks_of(p.gs, p.passes, true);
   }
   if (chunks > UINT32_MAX)
     return false;
-  *err = n ? launch_param(entries, n, uint32_t(chunks), 0, 0, s) : TEMPI_OK;
+  *err = n ? launch_param(entries, n, uint32_t(chunks), 0, tuned.shape.ctas_per_sm, s)
+           : TEMPI_OK;
   if (!*err && n)
     set_last_kernel("batch_copy");
+  counters().neighbor_unit++;
   return true;
 }
 
@@ -1227,15 +1263,9 @@ int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
   static std::vector<char> on_device; // the entries in the table
   static std::vector<CopyPair> pairs;
   std::lock_guard<std::mutex> l(mu);
-  std::unique_lock<std::mutex> tuning(g_tune_mu);
-  load_tuned_locked();
-  if (g_tuned.empty()) {
-    tuning.unlock();
-    int err;
-    if (run_single_objects(edges, n, s, &err))
-      return err;
-    tuning.lock();
-  }
+  int err;
+  if (run_single_objects(edges, n, s, &err))
+    return err;
   std::vector<tempi_copy_region> regions(static_cast<size_t>(n));
   for (int i = 0; i < n; ++i) {
     const CopyEdge &e = edges[i];
@@ -1243,21 +1273,17 @@ int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
                   e.dst_type->desc, e.src_count, e.dst_count};
   }
   uint64_t chunks = 0;
-  int err = build_pairs(regions.data(), n, &pairs, &chunks);
+  err = build_pairs(regions.data(), n, &pairs, &chunks);
   if (err || pairs.empty())
     return err;
   // a batch of a tuned signature takes the tuned choices
-  Shape shape;
-  auto it = g_tuned.empty() ? g_tuned.end() : g_tuned.find(signature(pairs, 0));
-  if (it != g_tuned.end()) {
-    shape = it->second.shape;
-    chunks = apply_passes(pairs, &it->second);
-  }
-  tuning.unlock();
+  Tuned tuned;
+  if (find_tuned(pairs.data(), pairs.size(), 0, &tuned))
+    chunks = apply_passes(pairs, &tuned);
+  const Shape shape = tuned.shape;
   const int count = int(pairs.size());
   const bool small = all_small(pairs);
-  if (small && count <= kParamRegions &&
-      (shape.threads == 0 || shape.threads == 256)) {
+  if (small && count <= kParamRegions && param_shape(shape)) {
     SmallPair entries[kParamRegions];
     for (int i = 0; i < count; ++i)
       entries[i] = make_small(pairs[i]);

@@ -84,7 +84,7 @@ extern "C" int64_t tempi_counter(const char *name) {
   C(recv_lib) C(isend_managed) C(irecv_managed) C(dispatch_hit)
   C(dispatch_miss) C(dispatch_measured) C(slab_hits) C(slab_misses) C(slab_bytes) C(slab_live_bytes) C(slab_cached_bytes) C(host_link_copies)
   C(send_contig_staged) C(recv_contig_staged) C(neighbor_fused)
-  C(neighbor_isir) C(neighbor_lib) C(neighbor_uploads) C(neighbor_tables) C(alltoallv_staged) C(alltoallv_remote_first)
+  C(neighbor_isir) C(neighbor_lib) C(neighbor_uploads) C(neighbor_tables) C(neighbor_unit) C(alltoallv_staged) C(alltoallv_remote_first)
   C(alltoallv_isir_staged) C(alltoallv_isir_remote_staged) C(alltoallv_lib)
 #undef C
   return -1;

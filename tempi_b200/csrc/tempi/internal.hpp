@@ -59,7 +59,7 @@ struct Counters {
   std::atomic<int64_t> host_link_copies{0};
   std::atomic<int64_t> send_contig_staged{0}, recv_contig_staged{0};
   std::atomic<int64_t> neighbor_fused{0}, neighbor_isir{0}, neighbor_lib{0},
-      neighbor_uploads{0}, neighbor_tables{0};
+      neighbor_uploads{0}, neighbor_tables{0}, neighbor_unit{0};
   std::atomic<int64_t> alltoallv_staged{0}, alltoallv_remote_first{0},
       alltoallv_isir_staged{0}, alltoallv_isir_remote_staged{0}, alltoallv_lib{0};
 };

@@ -94,3 +94,46 @@ def test_growing_exchanges_share_an_allocation(cuda, mpi_init):
         x.run()
         mpi.Comm_free(x.comm)
     assert _lib.counter("neighbor_tables") <= n + 1
+
+
+def test_single_objects_whatever_else_was_tuned(cuda, mpi_init, tmp_path, monkeypatch):
+    """Exchanges of up to 32 single objects take their entries from what the
+    types' commit settled, also after an unrelated batch was tuned; after a
+    batch of the same signature was tuned they take its choices."""
+    import torch
+
+    from tempi_b200 import halo
+
+    monkeypatch.setenv("TEMPI_CACHE_DIR", str(tmp_path))
+    _lib.tempi().tempi_reload_env()
+    other = halo.Grid((18, 11, 9), 1)
+    data = torch.from_numpy(H.splitmix_bytes(other.nbytes, 1)).cuda()
+    b = halo.HaloExchange([other], [data.data_ptr()])
+    b.tune(None, 1)
+    b.close()
+    t, extent = hvectors(24, [(3, 8), (2, 40)])
+    for edges in (1, 26, 32):
+        x = Exchange(t, extent, edges)
+        n = _lib.counter("neighbor_unit")
+        assert n >= 0
+        x.run()
+        x.run(8)
+        assert _lib.counter("neighbor_unit") == n + 2
+        mpi.Comm_free(x.comm)
+    # the signature of an exchange itself
+    g = halo.Grid((24, 16, 12), 2)
+    start = H.splitmix_bytes(g.nbytes, 2)
+    a, c = torch.from_numpy(start).cuda(), torch.from_numpy(start).cuda()
+    b = halo.HaloExchange([g], [a.data_ptr()])
+    b.tune(None, 2)
+    threads = b.config()[0]
+    b.launch()
+    n = _lib.counter("neighbor_unit")
+    torch.cuda.synchronize()
+    halo.exchange_alltoallw(halo.SelfGraph(g), c.data_ptr())
+    torch.cuda.synchronize()
+    assert _lib.counter("neighbor_unit") == n + (1 if threads == 256 else 0)
+    assert torch.equal(a, c)
+    b.close()
+    monkeypatch.undo()
+    _lib.tempi().tempi_reload_env()
