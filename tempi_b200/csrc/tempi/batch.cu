@@ -1195,7 +1195,8 @@ extern "C" int tempi_batch_create_copy(const tempi_copy_region *regions,
 namespace tempi {
 
 // The exchange of up to kParamRegions single objects whose two sides have at
-// most two strided dimensions (a halo's 26 regions): entries straight from the
+// most two strided dimensions (a halo's 26 regions), whatever number of edges
+// exchange nothing: entries straight from the
 // geometries settled when the types were committed, no division of lengths and
 // no descriptors copied (a 256^3 exchange: 4.1 us less host time a call, with
 // the types looked up under one lock).  An exchange whose own signature was
@@ -1204,11 +1205,14 @@ namespace tempi {
 // kernel.
 static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
                                int *err) {
-  if (n > kParamRegions)
-    return false;
   CopyPair pairs[kParamRegions];
+  int used = 0;
   for (int i = 0; i < n; ++i) {
     const CopyEdge &e = edges[i];
+    if (e.src_count == 0 && e.dst_count == 0)
+      continue;
+    if (used == kParamRegions)
+      return false;
     const TypeRecord &a = *e.src_type, &b = *e.dst_type;
     if (e.src_count != 1 || e.dst_count != 1 || !a.has_unit || !b.has_unit ||
         a.unit[4].nd > 2 || b.unit[4].nd > 2)
@@ -1219,15 +1223,15 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
                                    reinterpret_cast<uintptr_t>(dst)) |
                           a.unit[4].width | b.unit[4].width;
     const int k = __builtin_ctz(bits); // the width both sides prove: 2^k <= 16
-    pairs[i] = {src, dst, a.unit[k], b.unit[k], 0, 0};
+    pairs[used++] = {src, dst, a.unit[k], b.unit[k], 0, 0};
   }
   Tuned tuned;
-  const bool has_tuned = find_tuned(pairs, size_t(n), 0, &tuned);
+  const bool has_tuned = find_tuned(pairs, size_t(used), 0, &tuned);
   if (has_tuned && !param_shape(tuned.shape))
     return false;
   SmallPair entries[kParamRegions];
   uint64_t chunks = 0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = 0; i < used; ++i) {
     CopyPair &p = pairs[i];
     p.chunk_begin = uint32_t(chunks);
     p.passes = passes_of(region_class(p.gs), has_tuned ? &tuned : nullptr);
@@ -1236,9 +1240,10 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
   }
   if (chunks > UINT32_MAX)
     return false;
-  *err = n ? launch_param(entries, n, uint32_t(chunks), 0, tuned.shape.ctas_per_sm, s)
-           : TEMPI_OK;
-  if (!*err && n)
+  *err = used ? launch_param(entries, used, uint32_t(chunks), 0,
+                             tuned.shape.ctas_per_sm, s)
+              : TEMPI_OK;
+  if (!*err && used)
     set_last_kernel("batch_copy");
   counters().neighbor_unit++;
   return true;

@@ -137,3 +137,19 @@ def test_single_objects_whatever_else_was_tuned(cuda, mpi_init, tmp_path, monkey
     b.close()
     monkeypatch.undo()
     _lib.tempi().tempi_reload_env()
+
+
+@pytest.mark.parametrize("counts,single", [
+    ([1] * 25 + [0], True), ([0] * 5, True), ([0, 1] * 32, True), ([0] + [1] * 33, False),
+    ([1, 0, 2], False),
+])
+def test_edges_without_objects(cuda, mpi_init, counts, single):
+    """Neighbours that get nothing do not lengthen the others' way: only the
+    edges that exchange something count against the 32."""
+    t, extent = hvectors(24, [(3, 8), (2, 40)])
+    x = Exchange(t, extent, len(counts), counts, room=max(counts + [1]))
+    n = _lib.counter("neighbor_unit")
+    x.run()
+    x.run(8)
+    assert _lib.counter("neighbor_unit") == n + (2 if single else 0)
+    mpi.Comm_free(x.comm)
