@@ -154,8 +154,8 @@ int tempi_batch_destroy(tempi_batch *b);
    the batch on `stream` (`reps` launches per candidate, the L2 flushed
    before each; it allocates and frees a flush buffer of twice the L2),
    keeps the fastest choices for this batch, and remembers them for every
-   later batch with the same signature (the same region classes and sizes)
-   in this process and in TEMPI_CACHE_DIR/tempi_b200_batch_tune.txt.  It
+   later batch with the same signature (the same kernel, region classes and
+   sizes) in this process and in TEMPI_CACHE_DIR/tempi_b200_batch_tune.txt.  It
    drops a captured graph: capture again after tuning.  The reference has
    no counterpart (it packs one object per launch). */
 int tempi_batch_tune(tempi_batch *b, void *stream, int32_t reps);

@@ -706,14 +706,17 @@ uint64_t chunks_of(const Geometry &g, uint32_t passes, bool small) {
 // record, and its chunks, up to twice as many as the other kernels cut, can
 // be counted in 32 bits even at one pass each (so that no tuning of the
 // passes changes the answer).
-template <typename Rec> bool all_small(const std::vector<Rec> &recs) {
+template <typename Rec> bool all_small(const Rec *recs, size_t n) {
   uint64_t chunks = 0;
-  for (const Rec &r : recs) {
-    chunks += chunks_of(geometry_of(r), 1, true);
-    if (!is_small(r) || chunks > UINT32_MAX)
+  for (size_t i = 0; i < n; ++i) {
+    chunks += chunks_of(geometry_of(recs[i]), 1, true);
+    if (!is_small(recs[i]) || chunks > UINT32_MAX)
       return false;
   }
   return true;
+}
+template <typename Rec> bool all_small(const std::vector<Rec> &recs) {
+  return all_small(recs.data(), recs.size());
 }
 
 // warp chunks of every record, in order; the total (or more than
@@ -847,8 +850,13 @@ void load_tuned_locked() {
   std::fclose(f);
 }
 
-// signature of a batch: what kind of launch it is, and the multiset of its
-// records' (class, log2 words)
+// Signature of a batch: the kernels that run it, what kind of launch it is, and
+// the multiset of its records' (class, log2 words).  Choices hold for the
+// kernels that were timed: a pass of the compact ones is 4 words a lane, of the
+// others up to 8, and a different number of CTAs fits an SM.
+// kTunedKernels changes when either set's pass or occupancy does, so that a
+// tune file written before is left unused.
+constexpr uint32_t kTunedKernels = 2;
 template <typename Rec> uint64_t signature(const Rec *recs, size_t n, int unpack) {
   std::vector<uint32_t> keys;
   keys.reserve(n);
@@ -864,6 +872,8 @@ template <typename Rec> uint64_t signature(const Rec *recs, size_t n, int unpack
       h *= 1099511628211ull;
     }
   };
+  mix(kTunedKernels);
+  mix(all_small(recs, n));
   mix(std::is_same<Rec, CopyPair>::value ? 2u : uint32_t(unpack));
   for (uint32_t k : keys)
     mix(k);
