@@ -91,7 +91,8 @@ typedef struct tempi_desc {
    a thread per 16-B word of the destination; `unroll` = 1 or 4 words in
    flight per thread).  width: vector bytes for kernels 1, 2 and 4
    (1,2,4,8,16; never above what the alignment proof allows).
-   blocks_per_sm: resident blocks per SM the grid is sized for (kernel 4:
+   blocks_per_sm: resident blocks per SM the grid is sized for (0 between two
+   pinned host buffers: few enough to keep about 640 KB in flight; kernel 4:
    1..8; the 16 KB-chunk kernels run one warp per block, one block per SM
    for 96 MiB or more and 3 below, and blocks_per_sm only lowers that; the
    scattering unpack defaults to 3 for aligned copies of 32 MiB or more,
@@ -307,7 +308,8 @@ int64_t tempi_kernel_launches(void);
 /* name of the kernel variant the last tempi_pack/unpack used */
 const char *tempi_last_kernel(void);
 /* value of a named counter (reference include/counters.hpp groups):
-   "kernel_launches", "packs", "unpacks", "pack_bytes", "unpack_bytes",
+   "kernel_launches", "pack_ctas" (thread blocks of the word, row and shift
+   kernels' launches), "packs", "unpacks", "pack_bytes", "unpack_bytes",
    "lib_pack", "lib_unpack", "cached_types", "send_device", "send_oneshot",
    "send_staged", "send_lib", "recv_device", "recv_oneshot", "recv_staged",
    "recv_lib", "isend_managed", "irecv_managed", "dispatch_hit",

@@ -1410,7 +1410,10 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // 4-B words 182 at 1184, 151 at 96 to 148, 177 at 16.  So the grid holds
   // about 640 KB in flight, counting only the lanes that a row keeps busy
   // (64-B rows are bound by the number of requests and keep the full grid).
-  if (both_host) {
+  // A caller's own blocks_per_sm stands.
+  const bool asked_blocks =
+      cfg && cfg->blocks_per_sm > 0 && cfg->reserved != kOwnChoice;
+  if (both_host && !asked_blocks) {
     const int64_t n = g.block;
     const int64_t flight =
         kernel == 1   ? int64_t(threads) * kUnroll * g.width
@@ -1429,6 +1432,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   if (e != cudaSuccess)
     return cuda_error(e, "pack kernel launch");
   counters().kernel_launches++;
+  counters().pack_ctas += blocks;
   set_last_kernel(kernel_name(kernel, sel, unpack));
   return TEMPI_OK;
 }
