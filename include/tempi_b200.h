@@ -309,7 +309,8 @@ int64_t tempi_kernel_launches(void);
 const char *tempi_last_kernel(void);
 /* value of a named counter (reference include/counters.hpp groups):
    "kernel_launches", "pack_ctas" (thread blocks of the word, row and shift
-   kernels' launches), "packs", "unpacks", "pack_bytes", "unpack_bytes",
+   kernels' launches), "pointer_lookups" (buffers whose memory kind the
+   runtime was asked for), "packs", "unpacks", "pack_bytes", "unpack_bytes",
    "lib_pack", "lib_unpack", "cached_types", "send_device", "send_oneshot",
    "send_staged", "send_lib", "recv_device", "recv_oneshot", "recv_staged",
    "recv_lib", "isend_managed", "irecv_managed", "dispatch_hit",

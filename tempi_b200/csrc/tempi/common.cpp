@@ -78,7 +78,7 @@ extern "C" int64_t tempi_counter(const char *name) {
 #define C(x)                                                                   \
   if (n == #x)                                                                 \
     return c.x.load();
-  C(kernel_launches) C(pack_ctas) C(packs) C(unpacks) C(pack_bytes) C(unpack_bytes)
+  C(kernel_launches) C(pack_ctas) C(pointer_lookups) C(packs) C(unpacks) C(pack_bytes) C(unpack_bytes)
   C(lib_pack) C(lib_unpack) C(cached_types) C(send_device) C(send_oneshot)
   C(send_staged) C(send_lib) C(recv_device) C(recv_oneshot) C(recv_staged)
   C(recv_lib) C(isend_managed) C(irecv_managed) C(dispatch_hit)

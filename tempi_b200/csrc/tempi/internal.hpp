@@ -42,7 +42,7 @@ cudaError_t copy_complete(void *dst, const void *src, size_t n);
 
 // ---- counters (reference include/counters.hpp:14-115) ----------------------
 struct Counters {
-  std::atomic<int64_t> kernel_launches{0}, pack_ctas{0};
+  std::atomic<int64_t> kernel_launches{0}, pack_ctas{0}, pointer_lookups{0};
   std::atomic<int64_t> packs{0}, unpacks{0};
   std::atomic<int64_t> pack_bytes{0}, unpack_bytes{0};
   std::atomic<int64_t> lib_pack{0}, lib_unpack{0};

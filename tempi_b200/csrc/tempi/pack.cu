@@ -1242,6 +1242,28 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
                     int both_device) {
   const int sms = num_sms();
   int kernel = cfg ? cfg->kernel : 0;
+  // Where the buffers are, when the caller does not know: each is looked up at
+  // most once (0.1 us of a call's 3.1), and only if a rule below turns on it.
+  PtrInfo in_typed, in_packed;
+  bool typed_known = false, packed_known = false;
+  auto typed_info = [&]() -> const PtrInfo & {
+    if (!typed_known)
+      in_typed = classify(strided), typed_known = true;
+    return in_typed;
+  };
+  auto packed_info = [&]() -> const PtrInfo & {
+    if (!packed_known)
+      in_packed = classify(packed), packed_known = true;
+    return in_packed;
+  };
+  auto on_device = [&] {
+    return both_device >= 0 ? both_device == 1
+                            : typed_info().is_device && packed_info().is_device;
+  };
+  auto on_host = [&] {
+    return both_device >= 0 ? both_device == kBothHost
+                            : typed_info().is_host && packed_info().is_host;
+  };
   const bool cut = unpack && cuts_sectors(g, strided);
   if (kernel == 5 && g.block >= kRealignMinRow)
     return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
@@ -1250,13 +1272,10 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // by the dispatcher
   const bool own = kernel < 1 || kernel > 5 || cfg->reserved == kOwnChoice;
   if (own && realign_wins(g, uint64_t(g.rows) * uint64_t(g.block), unpack, cut,
-                          sms)) {
-    if (both_device < 0)
-      both_device = classify(strided).is_device && classify(packed).is_device;
-    if (both_device == 1)
-      return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
-                            cfg, stream);
-  }
+                          sms) &&
+      on_device())
+    return launch_realign(g, const_cast<char *>(strided), packed, unpack, cut,
+                          cfg, stream);
   // A staged kernel's bytes go through shared memory before the first store:
   // about 1.2 us more latency, which long streams make up for and a call that
   // is waited for does not below 16 MB (8 MB for rows below 64 B).  Where the
@@ -1271,9 +1290,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
       g.width >= (!unpack ? 16u : g.block < 64 ? 8u : 4u) &&
       uint64_t(g.rows) * uint64_t(g.block) <
           (g.block < 64 ? kStagedMinBytes / 2 : kStagedMinBytes) &&
-      (both_device >= 0
-           ? both_device == 1
-           : classify(strided).is_device && classify(packed).is_device)) {
+      on_device()) {
     kernel = 1;
     cfg = nullptr; // its launch shape is the staged kernel's
   }
@@ -1292,10 +1309,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
       bytes % 16 == 0 &&
       (unpack ? (reinterpret_cast<uintptr_t>(packed) & 15) == 0
               : g.width == 16) &&
-      (both_device >= 0
-           ? both_device == 1
-           : classify(strided).is_device && classify(packed).is_device) &&
-      staged_channel(stream);
+      on_device() && staged_channel(stream);
   // packs, and unpacks of wide aligned rows, run the bulk kernels
   BulkFn bulk = nullptr;
   if (staged &&
@@ -1348,11 +1362,8 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
     else
       kernel = 1;
   }
-  if (both_device < 0 && bytes >= kLinkMinBytes) {
-    const PtrInfo a = classify(strided), b = classify(packed);
-    both_device = a.is_device && b.is_device ? 1 : a.is_host && b.is_host ? kBothHost : 0;
-  }
-  const bool both_host = both_device == kBothHost;
+  // objects too small for the grids below to differ are not looked up for them
+  const bool placed = both_device >= 0 || bytes >= kLinkMinBytes;
   // rows per group of lanes for the shift kernel
   uint32_t lanes = 32;
   if (kernel == 3) {
@@ -1381,8 +1392,8 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   const bool own_shape =
       !cfg || cfg->reserved == kOwnChoice || !(cfg->threads || cfg->blocks_per_sm);
   const bool once = (kernel == 3 || (kernel == 2 && bytes >= kOnceRowsBytes)) &&
-                    both_device == 1 && own_shape && g.block >= kOnceMinRow &&
-                    g.block < kOnceMaxRow;
+                    own_shape && g.block >= kOnceMinRow &&
+                    g.block < kOnceMaxRow && placed && on_device();
   if (once)
     threads = 128;
   int64_t need;
@@ -1398,7 +1409,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
     // bytes 15.7 us against 16.8).
     const int64_t words = g.total_words;
     need = (words + threads * kUnroll - 1) / (threads * kUnroll);
-    if (both_device == 1)
+    if (need < sms && placed && on_device())
       need = std::max(need, std::min<int64_t>((words + threads - 1) / threads, sms));
   }
   int64_t blocks = once ? need : std::min<int64_t>(need, int64_t(sms) * bps);
@@ -1413,14 +1424,16 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // A caller's own blocks_per_sm stands.
   const bool asked_blocks =
       cfg && cfg->blocks_per_sm > 0 && cfg->reserved != kOwnChoice;
-  if (both_host && !asked_blocks) {
+  if (!asked_blocks && placed) {
     const int64_t n = g.block;
     const int64_t flight =
         kernel == 1   ? int64_t(threads) * kUnroll * g.width
         : kernel == 2 ? threads / 32 * std::min<int64_t>(n, 32 * kUnroll * g.width)
                       : threads / int(lanes) *
                             std::min<int64_t>(n, lanes * kShiftWords * 16);
-    blocks = std::min<int64_t>(blocks, (int64_t(640) << 10) / flight);
+    const int64_t most = (int64_t(640) << 10) / flight;
+    if (blocks > most && on_host())
+      blocks = most;
   }
   blocks = std::max<int64_t>(blocks, 1);
   const uint32_t sel = kernel == 3 ? lanes : g.width;

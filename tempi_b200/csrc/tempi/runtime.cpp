@@ -143,6 +143,7 @@ PtrInfo classify(const void *p) {
   PtrInfo info;
   if (!p || !cuda_available())
     return info;
+  counters().pointer_lookups++;
   cudaPointerAttributes a{};
   cudaError_t e = cudaPointerGetAttributes(&a, p);
   if (e != cudaSuccess) {
