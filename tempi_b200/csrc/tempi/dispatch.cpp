@@ -17,8 +17,8 @@
 
 namespace tempi {
 
-// the kernel configurations the model scores (outputs 0..9), measured and
-// launched as the dispatcher's own choice (kOwnChoice)
+// the kernel configurations the model scores (outputs 0..9), launched as the
+// dispatcher's own choice (kOwnChoice)
 const tempi_config kCandidates[kNumConfigs] = {
     {1, 0, 256, 0, 0, kOwnChoice},  // word kernel, 256 threads
     {1, 0, 512, 0, 0, kOwnChoice},  // word kernel, 512 threads
@@ -32,7 +32,33 @@ const tempi_config kCandidates[kNumConfigs] = {
     {4, 0, 256, 0, 8, kOwnChoice},  // staged kernel, 8 CTAs per SM
 };
 
+tempi_config measured_candidate(int k) {
+  tempi_config c = kCandidates[k];
+  c.reserved = kByName;
+  return c;
+}
+
 namespace {
+
+// What choose_config keeps for a layout: -1 the fixed rules, k a candidate that
+// the cost model picked, kNumConfigs + k one that was measured.
+tempi_config config_of(int choice) {
+  return choice < 0             ? tempi_config{}
+         : choice < kNumConfigs ? kCandidates[choice]
+                                : measured_candidate(choice - kNumConfigs);
+}
+
+// the choice that a measurement makes: the fastest candidate, or the fixed
+// rules where they are faster still (they reach kernels that no candidate
+// names)
+int fastest(const float *t, int lo, int fixed) {
+  int best = -1;
+  float least = std::isfinite(t[fixed]) ? t[fixed] : INFINITY;
+  for (int j = 0; j < kNumConfigs; ++j)
+    if (std::isfinite(t[lo + j]) && t[lo + j] < least)
+      best = kNumConfigs + j, least = t[lo + j];
+  return best;
+}
 
 float lg(double v) { return v > 0 ? float(std::log2(v)) : 0.f; }
 
@@ -445,7 +471,7 @@ tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
     auto it = r.configs.find(key); // every call after the first: no strings
     if (it != r.configs.end()) {
       counters().dispatch_hit++;
-      return it->second < 0 ? tempi_config{} : kCandidates[it->second];
+      return config_of(it->second);
     }
   }
   const std::string lkey =
@@ -458,7 +484,7 @@ tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
     if (lt != g_layouts.end()) {
       counters().dispatch_hit++;
       r.configs[key] = lt->second;
-      return lt->second < 0 ? tempi_config{} : kCandidates[lt->second];
+      return config_of(lt->second);
     }
   }
   counters().dispatch_miss++;
@@ -491,23 +517,16 @@ tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
       (mode == Dispatch::LEARNED && range == Range::MEASURE)) {
     counters().dispatch_measured++;
     float t[kMeasured];
-    const int me = measure_candidates(r.desc, incount, src_host, dst_host, 1, 2, t);
+    const int me = measure_candidates(r.desc, incount, src_host, dst_host,
+                                      kMeasureKernels | kMeasureNamed, 2, t);
     // a choice made at run time holds no scratch memory afterwards (its
     // buffers are the size of the layout's span)
     measure_release();
     if (me == TEMPI_OK) {
-      int best = -1;
-      for (int j = 0; j < kNumConfigs; ++j)
-        if (std::isfinite(t[lo + j]) && (best < 0 || t[lo + j] < t[lo + best]))
-          best = j;
-      choice = best;
+      choice = fastest(t, lo, unpack ? kFixedUnpack : kFixedPack);
       // the same measurement answers the other direction too
-      int other = -1;
-      const int lo2 = unpack ? kPackOut : kUnpackOut;
-      for (int j = 0; j < kNumConfigs; ++j)
-        if (std::isfinite(t[lo2 + j]) &&
-            (other < 0 || t[lo2 + j] < t[lo2 + other]))
-          other = j;
+      const int other = unpack ? fastest(t, kPackOut, kFixedPack)
+                               : fastest(t, kUnpackOut, kFixedUnpack);
       std::lock_guard<std::mutex> l(g_mu);
       r.configs[config_key(incount, src_host, dst_host, !unpack)] = other;
       remember_layout(lkey2, other);
@@ -516,7 +535,7 @@ tempi_config choose_config(TypeRecord &r, int64_t incount, bool src_host,
   std::lock_guard<std::mutex> l(g_mu);
   r.configs[key] = choice;
   remember_layout(lkey, choice);
-  return choice < 0 ? tempi_config{} : kCandidates[choice];
+  return config_of(choice);
 }
 
 Method choose_method(TypeRecord &r, int count) {

@@ -24,6 +24,9 @@ constexpr int kPackOut = 0, kUnpackOut = kNumConfigs,
               kMethodOut = 2 * kNumConfigs;
 static_assert(kMethodOut + kNumMethods == TEMPI_MLP_OUT, "model outputs");
 extern const tempi_config kCandidates[kNumConfigs];
+// candidate k as a measurement times and launches it: the kernel it names, no
+// other in its place
+tempi_config measured_candidate(int k);
 // measured entries: the model's outputs, then the fixed rules' pack and
 // unpack times (the policy without the model)
 constexpr int kFixedPack = TEMPI_MLP_OUT, kFixedUnpack = TEMPI_MLP_OUT + 1;
@@ -71,7 +74,10 @@ void dispatch_init();
 // Time every candidate: times_us[0..9] = pack and [10..19] = unpack with
 // each kernel configuration, [20..22] = self-send round trip by each method,
 // [23] / [24] = pack / unpack by the fixed rules (NaN where not measured).
-// `what`: bit 0 configurations, bit 1 methods.
+// `what`: kernel configurations, methods; the configurations as the cost
+// model's picks launch them (a rule may put another kernel in their place), or
+// the kernels that they name.
+constexpr int kMeasureKernels = 1, kMeasureMethods = 2, kMeasureNamed = 4;
 int measure_candidates(const tempi_desc &d, int64_t incount, bool src_host,
                        bool dst_host, int what, int reps, float *times_us);
 // Free the scratch buffers measure_candidates keeps between calls (the

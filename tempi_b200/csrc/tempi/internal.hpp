@@ -125,10 +125,16 @@ int make_geometry(const tempi_desc *d, int64_t incount, uintptr_t strided_base,
                   uintptr_t packed_base, int max_width, Geometry *g,
                   bool *empty);
 
-// tempi_config::reserved of a configuration the dispatcher chose: the launch
-// may still take the realign kernel (pack.cu realign_wins), which is not among
-// the candidates the cost model scores.
+// tempi_config::reserved of a configuration that the library chose, whose
+// launch shape is therefore the library's too.  kOwnChoice, the cost model's:
+// the launch may still take a kernel that is not among the candidates the
+// model scores, or that its rules prefer (pack.cu launch_geometry).
+// kByName: the kernel was timed on this layout against those rules, and runs.
 constexpr int32_t kOwnChoice = 0x7e91;
+constexpr int32_t kByName = 0x7e92;
+inline bool library_chose(const tempi_config &c) {
+  return c.reserved == kOwnChoice || c.reserved == kByName;
+}
 
 // Launch one pack (unpack=false) or unpack on `stream`.  both_device: 1 when
 // the caller knows both buffers are device memory proper, kBothHost when it

@@ -130,7 +130,7 @@ int measure_candidates(const tempi_desc &d, int64_t incount, bool src_host,
     return set_error(TEMPI_ERR_NO_MEM, "measure: scratch allocation failed");
   char *t_dev = static_cast<char *>(dev_view(typed, src_host));
   char *p_dev = static_cast<char *>(dev_view(pk, dst_host));
-  if (what & 1) {
+  if (what & kMeasureKernels) {
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
@@ -159,7 +159,10 @@ int measure_candidates(const tempi_desc &d, int64_t incount, bool src_host,
       const int k = i == 0 ? -1 : i - 1; // -1: the fixed rules
       if (k >= 0 && !eligible(d, incount, k))
         continue;
-      const tempi_config *cfg = k < 0 ? nullptr : &kCandidates[k];
+      const tempi_config named = k < 0 ? tempi_config{} : measured_candidate(k);
+      const tempi_config *cfg = k < 0                    ? nullptr
+                                : what & kMeasureNamed ? &named
+                                                       : &kCandidates[k];
       for (int u = 0; u < 2; ++u) {
         float t = pass(cfg, u == 1, 1);
         if (t <= 3 * best[u])
@@ -180,7 +183,7 @@ int measure_candidates(const tempi_desc &d, int64_t incount, bool src_host,
       return set_error(TEMPI_ERR_TIMEOUT,
                        "measure: a staged kernel gave up on its bulk copies");
   }
-  if ((what & 2) && !src_host && incount <= INT32_MAX) {
+  if ((what & kMeasureMethods) && !src_host && incount <= INT32_MAX) {
     void *typed2 = get(g_typed2, size_t(span), false);
     if (!typed2)
       return set_error(TEMPI_ERR_NO_MEM, "measure: scratch allocation failed");

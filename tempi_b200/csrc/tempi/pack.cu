@@ -1390,7 +1390,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // less (0.97 to 1.02); below 64 B a CTA's rows are too little work (0.94).
   // CTAs of 256 threads, as many as needed: 0.95 to 1.0, but for unpacks.
   const bool own_shape =
-      !cfg || cfg->reserved == kOwnChoice || !(cfg->threads || cfg->blocks_per_sm);
+      !cfg || library_chose(*cfg) || !(cfg->threads || cfg->blocks_per_sm);
   const bool once = (kernel == 3 || (kernel == 2 && bytes >= kOnceRowsBytes)) &&
                     own_shape && g.block >= kOnceMinRow &&
                     g.block < kOnceMaxRow && placed && on_device();
@@ -1423,7 +1423,7 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // (64-B rows are bound by the number of requests and keep the full grid).
   // A caller's own blocks_per_sm stands.
   const bool asked_blocks =
-      cfg && cfg->blocks_per_sm > 0 && cfg->reserved != kOwnChoice;
+      cfg && cfg->blocks_per_sm > 0 && !library_chose(*cfg);
   if (!asked_blocks && placed) {
     const int64_t n = g.block;
     const int64_t flight =
