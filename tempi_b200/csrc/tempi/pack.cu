@@ -1419,8 +1419,11 @@ int launch_geometry(const Geometry &g, const char *strided, char *packed,
   // and the two directions run one after the other: 1-KiB rows 159 us at 1184
   // CTAs, 143 at 148, 122 at 8 to 32 (16-B words, 256 threads); 256-B rows of
   // 4-B words 182 at 1184, 151 at 96 to 148, 177 at 16.  So the grid holds
-  // about 640 KB in flight, counting only the lanes that a row keeps busy
-  // (64-B rows are bound by the number of requests and keep the full grid).
+  // about 640 KB in flight; in the row and shift kernels only the lanes that a
+  // row keeps busy count (the shift kernel at 8 lanes on 64-B rows: 263 us on
+  // this grid, 363 on fewer CTAs).  The word kernel's are busy at any row:
+  // 65,536 rows of 64 B pack / unpack in 159 / 152 us on 40 CTAs of 16-B words,
+  // 169 / 155 on the full grid.
   // A caller's own blocks_per_sm stands.
   const bool asked_blocks =
       cfg && cfg->blocks_per_sm > 0 && !library_chose(*cfg);
