@@ -270,7 +270,8 @@ int tempi_features(const tempi_desc *d, int64_t incount, int typed_host,
    exhaustive autotuner; reference bin/measure_system.cpp,
    src/internal/measure_system.cu:381-610).  what: bit 0 configurations,
    bit 1 methods, bit 2 (with bit 0) the kernels that the configurations
-   name, as TEMPI_DISPATCH=exhaustive times them; without it what the cost
+   name, one launch at a time, as TEMPI_DISPATCH=exhaustive times them;
+   without it what the cost
    model's pick of each would launch, which the library's rules may replace.  times_us[TEMPI_MEASURED]: the twenty-three candidates above,
    then the fixed rules' (no model) pack and unpack; NaN where not
    measured. */
