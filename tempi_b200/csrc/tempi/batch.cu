@@ -880,19 +880,17 @@ template <typename Rec> uint64_t signature(const Rec *recs, size_t n, int unpack
   return h;
 }
 
-// passes of a region class from `t` (or the default)
-uint32_t passes_of(int cls, const Tuned *t) {
-  return t && t->passes[cls] ? t->passes[cls] : default_passes(cls);
+bool anything_tuned() {
+  std::lock_guard<std::mutex> l(g_tune_mu);
+  load_tuned_locked();
+  return !g_tuned.empty();
 }
 
-// The choices tuned for this signature, if any; no signature is formed while
-// nothing is tuned at all.
+// the choices tuned for this signature, if any
 template <typename Rec>
 bool find_tuned(const Rec *recs, size_t n, int unpack, Tuned *out) {
   std::lock_guard<std::mutex> l(g_tune_mu);
   load_tuned_locked();
-  if (g_tuned.empty())
-    return false;
   auto it = g_tuned.find(signature(recs, n, unpack));
   if (it == g_tuned.end())
     return false;
@@ -900,11 +898,13 @@ bool find_tuned(const Rec *recs, size_t n, int unpack, Tuned *out) {
   return true;
 }
 
-// the passes of every record and the chunk count
+// the passes of every record from `t` (or the defaults) and the chunk count
 template <typename Rec>
 uint64_t apply_passes(std::vector<Rec> &recs, const Tuned *t) {
-  for (Rec &r : recs)
-    r.passes = passes_of(region_class(geometry_of(r)), t);
+  for (Rec &r : recs) {
+    const int c = region_class(geometry_of(r));
+    r.passes = t && t->passes[c] ? t->passes[c] : default_passes(c);
+  }
   return assign_chunks(recs);
 }
 
@@ -1204,6 +1204,38 @@ extern "C" int tempi_batch_create_copy(const tempi_copy_region *regions,
 
 namespace tempi {
 
+// the pair of an edge of single objects
+static CopyPair unit_pair(const CopyEdge &e, uint32_t chunk_begin) {
+  const TypeRecord &a = *e.src_type, &b = *e.dst_type;
+  const char *src = e.src_origin + a.desc.start;
+  char *dst = e.dst_origin + b.desc.start;
+  const uint32_t bits = uint32_t(reinterpret_cast<uintptr_t>(src) |
+                                 reinterpret_cast<uintptr_t>(dst)) |
+                        a.unit[4].width | b.unit[4].width;
+  const int k = __builtin_ctz(bits); // the width both sides prove: 2^k <= 16
+  return {src, dst, a.unit[k], b.unit[k], chunk_begin, 0};
+}
+
+// The entries of single objects at the choices tuned for their signature, if
+// any; false when those need another kernel.  (Kept out of the loop that forms
+// the entries: processes that tuned nothing do not pay for it.)
+__attribute__((noinline)) static bool take_tuned(const CopyEdge *edges, int n,
+                                                 SmallPair *entries,
+                                                 uint64_t *chunks, Tuned *tuned) {
+  std::vector<CopyPair> pairs;
+  for (int i = 0; i < n; ++i)
+    if (edges[i].src_count)
+      pairs.push_back(unit_pair(edges[i], 0));
+  if (!find_tuned(pairs.data(), pairs.size(), 0, tuned))
+    return true;
+  if (!param_shape(tuned->shape))
+    return false;
+  *chunks = apply_passes(pairs, tuned);
+  for (size_t i = 0; i < pairs.size(); ++i)
+    entries[i] = make_small(pairs[i]);
+  return true;
+}
+
 // The exchange of up to kParamRegions single objects whose two sides have at
 // most two strided dimensions (a halo's 26 regions), whatever number of edges
 // exchange nothing: entries straight from the
@@ -1215,8 +1247,9 @@ namespace tempi {
 // kernel.
 static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
                                int *err) {
-  CopyPair pairs[kParamRegions];
+  SmallPair entries[kParamRegions];
   int used = 0;
+  uint64_t chunks = 0;
   for (int i = 0; i < n; ++i) {
     const CopyEdge &e = edges[i];
     if (e.src_count == 0 && e.dst_count == 0)
@@ -1227,27 +1260,14 @@ static bool run_single_objects(const CopyEdge *edges, int n, cudaStream_t s,
     if (e.src_count != 1 || e.dst_count != 1 || !a.has_unit || !b.has_unit ||
         a.unit[4].nd > 2 || b.unit[4].nd > 2)
       return false;
-    const char *src = e.src_origin + a.desc.start;
-    char *dst = e.dst_origin + b.desc.start;
-    const uint32_t bits = uint32_t(reinterpret_cast<uintptr_t>(src) |
-                                   reinterpret_cast<uintptr_t>(dst)) |
-                          a.unit[4].width | b.unit[4].width;
-    const int k = __builtin_ctz(bits); // the width both sides prove: 2^k <= 16
-    pairs[used++] = {src, dst, a.unit[k], b.unit[k], 0, 0};
-  }
-  Tuned tuned;
-  const bool has_tuned = find_tuned(pairs, size_t(used), 0, &tuned);
-  if (has_tuned && !param_shape(tuned.shape))
-    return false;
-  SmallPair entries[kParamRegions];
-  uint64_t chunks = 0;
-  for (int i = 0; i < used; ++i) {
-    CopyPair &p = pairs[i];
-    p.chunk_begin = uint32_t(chunks);
-    p.passes = passes_of(region_class(p.gs), has_tuned ? &tuned : nullptr);
-    entries[i] = make_small(p);
+    CopyPair p = unit_pair(e, uint32_t(chunks));
+    p.passes = default_passes(region_class(p.gs));
+    entries[used++] = make_small(p);
     chunks += chunks_of(p.gs, p.passes, true);
   }
+  Tuned tuned;
+  if (anything_tuned() && !take_tuned(edges, n, entries, &chunks, &tuned))
+    return false;
   if (chunks > UINT32_MAX)
     return false;
   *err = used ? launch_param(entries, used, uint32_t(chunks), 0,
@@ -1293,7 +1313,7 @@ int copy_batch_run(const CopyEdge *edges, int n, cudaStream_t s) {
     return err;
   // a batch of a tuned signature takes the tuned choices
   Tuned tuned;
-  if (find_tuned(pairs.data(), pairs.size(), 0, &tuned))
+  if (anything_tuned() && find_tuned(pairs.data(), pairs.size(), 0, &tuned))
     chunks = apply_passes(pairs, &tuned);
   const Shape shape = tuned.shape;
   const int count = int(pairs.size());
